@@ -309,7 +309,7 @@ def work(case):
     kind = case["kind"]
     nen = (case["p"] + 1) ** case["dim"]
     # the symmetric half of sum_q w G^T G per cell; every value written once
-    asm_flops = cells * nen * nen * (case["dim"] * B) ** (2 if B > 1 else 1) * nen
+    asm_flops = cells * nen * nen * case["dim"] * B * nen
     asm_bytes = pairs * B * B * 8 + 24 * dofs // B + 4 * nen * cells + 8 * dofs
     val = 4 if case.get("prec") == "mixed" else 8
     step = _spmv_bytes(case, val) + 72 * dofs
