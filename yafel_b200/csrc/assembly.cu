@@ -16,13 +16,15 @@
 // (CGAssembly.hpp:149-156).
 //
 // Values: cells are coloured on the host so that cells of one colour share no
-// node; one launch per colour, one CTA per cell.  The CTA computes the Jacobian,
-// jxw and physical gradients of every quadrature point into shared memory, then
-// each thread owns node pairs (A,B) of the element matrix, accumulates their
-// dpn x dpn blocks over the quadrature points in registers and adds them into
-// the global values (binary search of the column in the row).  No floating-point
-// atomics: colours in ascending order fix the summation order, so assembly is
-// deterministic.
+// node; one launch per colour.  Every warp takes a cell of its own: the inverse
+// Jacobians of its quadrature points go to shared memory, the element matrix is
+// formed in 8x8-node tiles by FP64 matrix instructions from the reference
+// gradients (one table per CTA), and the tiles are added into the global values.
+// No floating-point races: colours in ascending order fix the summation order, so
+// assembly is deterministic.  Where an entry lies, and
+// whether the cell is the first to touch it, comes from a scatter map laid out
+// with the pattern (16 bits per element entry): first touches are plain stores,
+// so the values are neither cleared nor read before.
 #include "internal.h"
 #include "device_common.cuh"
 #include "host_fe.h"
@@ -41,6 +43,10 @@ struct ElementGroup {
     double *d_tab = nullptr;        // N (nq*nen) | dN (nq*nen*dim) | w (nq)
     int32_t *d_order = nullptr;     // cells sorted by colour
     std::vector<int32_t> color_ptr; // colour c -> [color_ptr[c], color_ptr[c+1])
+    // scatter map, nen*nen entries per cell in the order of d_order: bits 0..14 the
+    // entry's position in its node row, bit 15 set when no earlier cell (group, then
+    // colour) touches it; NULL when it could not be built (see build_pattern)
+    uint16_t *d_map = nullptr;
 };
 
 struct yg_dofmap_t {
@@ -195,26 +201,98 @@ k_row_count(int32_t nnodes, const int64_t *__restrict__ aptr, const int32_t *__r
     }
 }
 
+// Where the cells of an assembly group stand: position in the group's colour
+// order and rank (64 * group + colour), by which cells of one node are told apart.
+__global__ void k_cell_slots(const int32_t *__restrict__ order, int n, int first, int rank, int32_t *__restrict__ slot,
+                             uint8_t *__restrict__ ranks) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        slot[order[t]] = first + t;
+        ranks[order[t]] = (uint8_t)rank;
+    }
+}
+
+struct ScatterMaps {
+    const int32_t *slot = nullptr;   // per cell, k_cell_slots
+    const uint8_t *rank = nullptr;
+    uint16_t *map[2] = {nullptr, nullptr};  // per group
+    int nen[2] = {0, 0};
+};
+
+// Rows of the node graph and, when `sm.slot` is given, the scatter map entries of
+// the row's node in each of its cells: the warp holds the row's sorted columns in
+// shared memory, marks each column with the lowest rank that touches it, and
+// writes every (cell, local node) pair's position with the first-touch bit.
+// *odd is set when a cell does not list exactly its element's nodes, each once;
+// the map is then not used.
 __global__ void __launch_bounds__(kRowWarps * 32)
 k_row_fill(int32_t nnodes, const int64_t *__restrict__ aptr, const int32_t *__restrict__ adj,
            const int32_t *__restrict__ off, const int32_t *__restrict__ el, const int64_t *__restrict__ rowptr64,
-           int32_t *__restrict__ rowptr, int32_t *__restrict__ col) {
+           int32_t *__restrict__ rowptr, int32_t *__restrict__ col, ScatterMaps sm, int32_t *__restrict__ odd) {
     __shared__ int32_t sbuf[kRowWarps][kRowCap];
+    __shared__ uint8_t smin[kRowWarps][kRowCap];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int64_t node = blockIdx.x * (int64_t)kRowWarps + w; node < nnodes; node += (int64_t)gridDim.x * kRowWarps) {
         int32_t *buf = sbuf[w];
+        uint8_t *low = smin[w];
         int u = row_unique((int)node, aptr, adj, off, el, buf);
+        const int64_t a0 = aptr[node], a1 = aptr[node + 1];
         int cnt = 0;
-        for (int64_t a = aptr[node]; a < aptr[node + 1]; ++a) cnt += off[adj[a] + 1] - off[adj[a]];
+        for (int64_t a = a0; a < a1; ++a) cnt += off[adj[a] + 1] - off[adj[a]];
         int64_t base = rowptr64[node];
         if (lane == 0) rowptr[node] = (int32_t)base;
+        // compact the unique columns to the front of the buffer and write them out
         int written = 0;
         for (int i0 = 0; i0 < cnt && u >= 0; i0 += 32) {
             int i = i0 + lane;
-            bool keep = i < cnt && (i == 0 || buf[i] != buf[i - 1]);
+            const int v = i < cnt ? buf[i] : 0;
+            bool keep = i < cnt && (i == 0 || v != buf[i - 1]);
             unsigned m = __ballot_sync(0xffffffffu, keep);
-            if (keep) col[base + written + __popc(m & ((1u << lane) - 1))] = buf[i];
+            __syncwarp();
+            if (keep) {
+                const int k = written + __popc(m & ((1u << lane) - 1));
+                col[base + k] = v;
+                buf[k] = v;
+                low[k] = 255;
+            }
             written += __popc(m);
+            __syncwarp();
+        }
+        if (sm.slot && u >= 0) {
+            auto position = [&](int c) {
+                int lo = 0, hi = written - 1;
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    if (buf[mid] < c) lo = mid + 1; else hi = mid;
+                }
+                return lo;
+            };
+            for (int pass = 0; pass < 2; ++pass)
+                for (int64_t a = a0; a < a1; ++a) {
+                    const int c = adj[a], b = off[c], nen = off[c + 1] - b;
+                    const uint8_t rk = sm.rank[c];
+                    const int g = rk >> 6;
+                    if (nen != sm.nen[g]) {
+                        if (lane == 0) *odd = 1;
+                        continue;
+                    }
+                    int self = -1, found = 0;
+                    for (int i0 = 0; i0 < nen; i0 += 32) {
+                        const unsigned m = __ballot_sync(0xffffffffu, i0 + lane < nen && el[b + i0 + lane] == (int32_t)node);
+                        if (m) self = i0 + __ffs(m) - 1;
+                        found += __popc(m);
+                    }
+                    if (found != 1) {
+                        if (lane == 0) *odd = 1;
+                        continue;
+                    }
+                    uint16_t *out = sm.map[g] + ((int64_t)sm.slot[c] * nen + self) * nen;
+                    for (int i = lane; i < nen; i += 32) {
+                        const int k = position(el[b + i]);
+                        if (pass == 0) low[k] = min(low[k], rk);
+                        else out[i] = (uint16_t)(k | (low[k] == rk ? 0x8000 : 0));
+                    }
+                    __syncwarp();
+                }
         }
         __syncwarp();
     }
@@ -255,53 +333,154 @@ __device__ __forceinline__ int find_col(const int32_t *__restrict__ col, int lo,
     return -1;
 }
 
-// Address of scalar entry (i,k) of node block (nA -> position pos in the node row).
-__device__ __forceinline__ int64_t entry_addr(int format, int D, const int32_t *__restrict__ nrp, int nA, int pos, int i,
-                                              int k) {
-    if (format == YG_FORMAT_BCSR) return (int64_t)pos * D * D + i * D + k;
-    int32_t rs = nrp[nA], len = nrp[nA + 1] - rs;
-    return (int64_t)rs * D * D + (int64_t)i * len * D + (int64_t)(pos - rs) * D + k;
+__device__ __forceinline__ void dmma8x8x4(double (&c)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+        : "+d"(c[0]), "+d"(c[1])
+        : "d"(a), "d"(b));
 }
 
-template <int NSD, int DPN, int PHYS>
-__global__ void __launch_bounds__(128)
-k_assemble(const int32_t *__restrict__ order, int ncell, const int32_t *__restrict__ off,
-           const int32_t *__restrict__ el, const double *__restrict__ nodes, const double *__restrict__ tab, int nen,
-           int nq, int tdim, PhysParams prm, const int32_t *__restrict__ nrp, const int32_t *__restrict__ ncol,
-           double *__restrict__ val, int format, double *__restrict__ residual, int want_K, int want_R) {
-    extern __shared__ double sm[];
-    double *xe = sm;                       // nen*3
-    double *G = xe + 3 * nen;              // nq*nen*NSD
-    double *jxw = G + (size_t)nq * nen * NSD;  // nq
-    double *Ji = jxw + nq;                 // nq*9
-    int32_t *gn = reinterpret_cast<int32_t *>(Ji + 9 * nq);  // nen
-    const double *tN = tab;
-    const double *tdN = tab + (size_t)nq * nen;
-    const double *tw = tdN + (size_t)nq * nen * tdim;
-    constexpr bool SYM = (PHYS != YG_SUPG);
+// Sizes of an element's tables.  Quadrature points are padded to a multiple of 4
+// (zero weights and gradients); a row of nodes has a stride of 4 or 12 modulo 16
+// doubles, so that the 4 points x 8 nodes of a matrix fragment fall into
+// different banks.
+__host__ __device__ inline int asm_points(int nq) { return (nq + 3) & ~3; }
+__host__ __device__ inline int asm_stride(int nen) {
+    int s = (nen + 3) & ~3;
+    while ((s & 15) != 4 && (s & 15) != 12) s += 4;
+    return s;
+}
+// The CTA's table of reference gradients, [direction][point][node]: row q of a
+// direction starts q / 4 doubles late, so that 16 points of one node (the lanes of
+// the Jacobian) fall into different banks too.
+__host__ __device__ inline int asm_plane(int nen, int nq) { return asm_points(nq) * asm_stride(nen) + asm_points(nq) / 4; }
+__host__ __device__ inline int asm_table_doubles(int nen, int nq, int nsd) { return (nsd * asm_plane(nen, nq) + 1) & ~1; }
+// doubles kept per quadrature point of a cell (even: read 16 bytes at a time): w
+// and, elasticity: the inverse Jacobian; Poisson: the upper triangle of w J^-1 J^-T;
+// SUPG: w J^-1 Kd J^-T, the advection and the load's upwind vectors in reference
+// directions
+__host__ __device__ constexpr int asm_coefs(int phys, int nsd) {
+    return (1 + (phys == YG_ELASTICITY ? nsd * nsd : phys == YG_POISSON ? nsd * (nsd + 1) / 2 : nsd * nsd + 2 * nsd) + 1) / 2 * 2;
+}
+// doubles of one warp's tile buffer: 64 blocks of E entries, a double more every 16 blocks
+__host__ __device__ constexpr int asm_tile_doubles(int E) { return E > 1 ? 64 * E + 4 : 0; }
+// doubles of one warp: coefficients | tile | node coordinates | rows (node, start, length; 3 ints each)
+__host__ __device__ inline int asm_warp_doubles(int nen, int nq, int nsd, int E, int phys) {
+    return (asm_points(nq) * asm_coefs(phys, nsd) + asm_tile_doubles(E) + 3 * nen + (3 * nen + 1) / 2 + 1) & ~1;
+}
+constexpr int kAsmWarps = 10;  // warps per CTA at most
 
-    for (int t = blockIdx.x; t < ncell; t += gridDim.x) {
-        const int c = order[t];
-        const int base = off[c];
-        for (int a = threadIdx.x; a < nen; a += blockDim.x) {
-            int n = el[base + a];
-            gn[a] = n;
-            xe[3 * a + 0] = nodes[3 * (int64_t)n + 0];
-            xe[3 * a + 1] = nodes[3 * (int64_t)n + 1];
-            xe[3 * a + 2] = nodes[3 * (int64_t)n + 2];
-        }
-        __syncthreads();
-        // Element::update: Jacobian, det, inverse per quadrature point
-        for (int q = threadIdx.x; q < nq; q += blockDim.x) {
-            double J[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-            for (int A = 0; A < nen; ++A) {
-                const double *d = tdN + ((size_t)q * nen + A) * tdim;
+// The cells order[0 .. ncell) of one colour; map points at the first one's
+// scatter entries (NULL: positions are searched and added to cleared values).
+//
+// The element matrix is M^ik[A][B] = sum_q w_q dN_A/dx_i dN_B/dx_k (elasticity:
+// K^ik = lambda M^ik + mu M^ki + mu delta_ik tr M), that is NSD x NSD products
+// G_i^T W G_k of nen x nq matrices; the scalar physics take dN_A^T T_q dN_B with the
+// 3x3 T_q of the point.  A warp takes an 8x8-node tile at a time and runs m8n8k4
+// FP64 matrix instructions over the quadrature points, 9 accumulators per tile in
+// 3D elasticity, so a lane ends with all (i, k) of its two node pairs.  A fragment
+// of physical gradients is formed on the way from the table of reference
+// gradients that the CTA's warps share: 21 vector FMAs beside 9 matrix
+// instructions, and a cell needs 8 KB of shared memory instead of 27.  Only tiles
+// on and above the diagonal are formed for the symmetric physics, the others are
+// the transposes.  Tiles of blocks go through shared memory so that the lanes of a
+// global access fall on consecutive entries of a block: 32 / E blocks at a time,
+// a lane keeping its entry of the block, so that a store costs a shuffle, a
+// shared load and one address.  An entry that an earlier cell has touched is
+// added to by a reduction that returns nothing (one cell per launch touches an
+// entry, so its order is that of the launches); nothing in the scatter waits for
+// memory, and no warp waits for another.
+//
+// Values alone (tangent; all colours), against a CTA per cell that formed every
+// entry by vector FMAs and read, added and wrote back the cleared values:
+// 33^3 Q2 hexahedra 3x3 blocks 2.81 -> 1.39 ms, 48^3 Q1 1.24 -> 0.41 ms, 14^3 Q3 5.29 ->
+// 1.82 ms, scalar 37^3 Q2 2.23 -> 0.71 ms, 60^3 Q1 1.53 -> 0.25 ms, 200^2 Q2 2x2 blocks
+// 0.33 -> 0.13 ms.  Floors of the first: 161k FMA per cell, 0.16 ms at the 37
+// TFLOP/s the matrix instructions reach; 26.2M block updates of 72 bytes, 18.6M of
+// them first touches, 0.37 ms.  What bounds it now is the shared-memory pipe (65 %
+// busy: fragments, and the tiles on their way out) at the 20 warps per SM that the
+// 36 accumulator registers leave.
+template <int NSD, int DPN, int PHYS, bool BCSR>
+__global__ void __launch_bounds__(32 * kAsmWarps, PHYS == YG_ELASTICITY ? 2 : 3)
+k_assemble(const int32_t *__restrict__ order, int ncell, const uint16_t *__restrict__ map,
+           const int32_t *__restrict__ off, const int32_t *__restrict__ el, const double *__restrict__ nodes,
+           const double *__restrict__ tab, int nen, int nq, PhysParams prm, const int32_t *__restrict__ nrp,
+           const int32_t *__restrict__ ncol, double *__restrict__ val, double *__restrict__ residual, int want_K,
+           int want_R) {
+    extern __shared__ __align__(16) double sm[];
+    constexpr bool SYM = (PHYS != YG_SUPG);
+    constexpr int NC = PHYS == YG_ELASTICITY ? NSD * NSD : 1;  // accumulators per tile
+    constexpr int E = DPN * DPN, CO = asm_coefs(PHYS, NSD);
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+    const int nqp = asm_points(nq), S = asm_stride(nen), plane = asm_plane(nen, nq);
+    double *T = sm;
+    double *coef = T + asm_table_doubles(nen, nq, NSD) + wib * asm_warp_doubles(nen, nq, NSD, E, PHYS);
+    double *tile = coef + nqp * CO;
+    double *xe = tile + asm_tile_doubles(E);
+    int32_t *ge = reinterpret_cast<int32_t *>(xe + 3 * nen);
+    const double *tN = tab;
+    const double *tdN = tab + nq * nen, *tw = tdN + nq * nen * NSD;
+    for (int i = threadIdx.x; i < nqp * nen; i += blockDim.x) {
+        const int q = i / nen, A = i - q * nen;
 #pragma unroll
-                for (int i = 0; i < NSD; ++i)
-#pragma unroll
-                    for (int j = 0; j < NSD; ++j) J[i][j] += xe[3 * A + i] * d[j];
+        for (int j = 0; j < NSD; ++j) T[j * plane + q * S + (q >> 2) + A] = q < nq ? tdN[i * NSD + j] : 0.0;
+    }
+    for (int i = nq * CO + lane; i < nqp * CO; i += 32) coef[i] = 0;
+    __syncthreads();
+
+    const int nteams = gridDim.x * nwarp, nt = (nen + 7) >> 3, ntiles = SYM ? nt * (nt + 1) / 2 : nt * nt;
+    int t = blockIdx.x * nwarp + wib;
+    // the lane's node of the next cell, fetched a cell ahead, one dependent load per step
+    int n = 0, r0 = 0, r1 = 0;
+    double x = 0, y = 0, z = 0;
+    if (t < ncell && lane < nen) {
+        n = el[off[order[t]] + lane];
+        r0 = nrp[n];
+        r1 = nrp[n + 1];
+        x = nodes[3 * (int64_t)n];
+        y = nodes[3 * (int64_t)n + 1];
+        z = nodes[3 * (int64_t)n + 2];
+    }
+    for (; t < ncell; t += nteams) {
+        auto put_node = [&](int a) {
+            xe[3 * a] = x;
+            xe[3 * a + 1] = y;
+            xe[3 * a + 2] = z;
+            ge[3 * a] = n;
+            ge[3 * a + 1] = r0;
+            ge[3 * a + 2] = r1 - r0;
+        };
+        if (lane < nen) put_node(lane);
+        if (nen > 32) {
+            const int base = off[order[t]];
+            for (int a = lane + 32; a < nen; a += 32) {
+                n = el[base + a];
+                r0 = nrp[n];
+                r1 = nrp[n + 1];
+                x = nodes[3 * (int64_t)n];
+                y = nodes[3 * (int64_t)n + 1];
+                z = nodes[3 * (int64_t)n + 2];
+                put_node(a);
             }
-            double det, inv[3][3];
+        }
+        const uint16_t *cmap = map ? map + (int64_t)t * nen * nen : nullptr;
+        if (map && want_K)
+            for (int i = 64 * lane; i < nen * nen; i += 64 * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(cmap + i));
+        const bool pre = t + nteams < ncell && lane < nen;
+        int next = 0;
+        if (pre) next = __ldg(order + t + nteams);
+        __syncwarp();
+        // Element::update, a lane per quadrature point: Jacobian, det, inverse
+        for (int q = lane; q < nq; q += 32) {
+            double J[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, inv[3][3], det;
+#pragma unroll 3
+            for (int A = 0; A < nen; ++A) {
+#pragma unroll
+                for (int j = 0; j < NSD; ++j) {
+                    const double d = T[j * plane + q * S + (q >> 2) + A];
+#pragma unroll
+                    for (int i = 0; i < NSD; ++i) J[i][j] += xe[3 * A + i] * d;
+                }
+            }
             if (NSD == 1) {
                 det = J[0][0];
                 inv[0][0] = 1.0 / J[0][0];
@@ -324,140 +503,302 @@ k_assemble(const int32_t *__restrict__ order, int ncell, const int32_t *__restri
                 inv[2][1] = -(J[0][0] * J[2][1] - J[2][0] * J[0][1]) * di;
                 inv[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) * di;
             }
-            jxw[q] = det * tw[q];
+            const double w = det * __ldg(tw + q);
+            double *c = coef + q * CO;
+            *c++ = w;
+            // dN/dx_d = sum_j inv[j][d] dN/dxi_j
+            if (PHYS == YG_ELASTICITY) {
 #pragma unroll
-            for (int i = 0; i < NSD; ++i)
+                for (int j = 0; j < NSD; ++j)
 #pragma unroll
-                for (int j = 0; j < NSD; ++j) Ji[9 * q + 3 * i + j] = inv[i][j];
-        }
-        __syncthreads();
-        // physical gradients dN/dx_d = sum_j Jinv(j,d) dN/dxi_j
-        for (int idx = threadIdx.x; idx < nq * nen; idx += blockDim.x) {
-            const int q = idx / nen;
-            const double *d = tdN + (size_t)idx * tdim;
+                    for (int d = 0; d < NSD; ++d) *c++ = inv[j][d];
+            } else if (PHYS == YG_POISSON) {
 #pragma unroll
-            for (int dd = 0; dd < NSD; ++dd) {
-                double s = 0;
+                for (int j = 0; j < NSD; ++j)
 #pragma unroll
-                for (int j = 0; j < NSD; ++j) s += Ji[9 * q + 3 * j + dd] * d[j];
-                G[(size_t)idx * NSD + dd] = s;
-            }
-        }
-        __syncthreads();
-        if (want_K) {
-            const int npairs = SYM ? nen * (nen + 1) / 2 : nen * nen;
-            for (int pr = threadIdx.x; pr < npairs; pr += blockDim.x) {
-                int A, B;
-                if (SYM) {  // pr -> (A <= B), row-major over the upper triangle
-                    A = 0;
-                    int rem = pr;
-                    while (rem >= nen - A) { rem -= nen - A; ++A; }
-                    B = A + rem;
-                } else {
-                    A = pr / nen;
-                    B = pr % nen;
-                }
-                double K[DPN][DPN];
-#pragma unroll
-                for (int i = 0; i < DPN; ++i)
-#pragma unroll
-                    for (int k = 0; k < DPN; ++k) K[i][k] = 0;
-                for (int q = 0; q < nq; ++q) {
-                    const double *gA = G + ((size_t)q * nen + A) * NSD;
-                    const double *gB = G + ((size_t)q * nen + B) * NSD;
-                    const double w = jxw[q];
-                    if (PHYS == YG_POISSON) {
-                        double dt = 0;
-#pragma unroll
-                        for (int d = 0; d < NSD; ++d) dt += gA[d] * gB[d];
-                        K[0][0] += prm.p[0] * (dt * w);
-                    } else if (PHYS == YG_ELASTICITY) {
-                        double a[NSD], b[NSD], dt = 0;
-#pragma unroll
-                        for (int d = 0; d < NSD; ++d) { a[d] = gA[d]; b[d] = gB[d]; dt += a[d] * b[d]; }
-                        const double sw = prm.p[0] * w, lam = prm.p[1], mu = prm.p[2];
-#pragma unroll
-                        for (int i = 0; i < NSD; ++i)
-#pragma unroll
-                            for (int k = 0; k < NSD; ++k)
-                                K[i][k] += sw * (lam * a[i] * b[k] + mu * ((i == k ? dt : 0.0) + a[k] * b[i]));
-                    } else {  // SUPG: advection summed NSD times, as the reference does
-                        const double NA = tN[(size_t)q * nen + A];
+                    for (int l = j; l < NSD; ++l) {
                         double s = 0;
 #pragma unroll
-                        for (int ac = 0; ac < NSD; ++ac)
+                        for (int d = 0; d < NSD; ++d) s += inv[j][d] * inv[l][d];
+                        *c++ = w * s;
+                    }
+            } else {
 #pragma unroll
-                            for (int bc = 0; bc < NSD; ++bc)
-                                s += NA * prm.U[bc] * gB[bc] + gA[ac] * gB[bc] * prm.Kd[3 * ac + bc];
-                        K[0][0] += s * w;
+                for (int j = 0; j < NSD; ++j) {
+                    double k[NSD];  // row j of J^-1 Kd
+#pragma unroll
+                    for (int e = 0; e < NSD; ++e) {
+                        k[e] = 0;
+#pragma unroll
+                        for (int d = 0; d < NSD; ++d) k[e] += inv[j][d] * prm.Kd[3 * d + e];
+                    }
+#pragma unroll
+                    for (int l = 0; l < NSD; ++l) {
+                        double s = 0;
+#pragma unroll
+                        for (int e = 0; e < NSD; ++e) s += k[e] * inv[l][e];
+                        *c++ = w * s;
                     }
                 }
-                const int nA = gn[A], nB = gn[B];
-                int rs = __ldg(nrp + nA), re = __ldg(nrp + nA + 1);
-                int pos = find_col(ncol, rs, re, nB);
-                if (pos >= 0) {
+                // advection (summed NSD times, as the reference does), then the load's upwind direction
 #pragma unroll
-                    for (int i = 0; i < DPN; ++i)
+                for (int l = 0; l < NSD; ++l) {
+                    double s = 0;
 #pragma unroll
-                        for (int k = 0; k < DPN; ++k) val[entry_addr(format, DPN, nrp, nA, pos, i, k)] += K[i][k];
+                    for (int d = 0; d < NSD; ++d) s += prm.U[d] * inv[l][d];
+                    *c++ = NSD * w * s;
                 }
-                if (SYM && A != B) {
-                    rs = __ldg(nrp + nB);
-                    re = __ldg(nrp + nB + 1);
-                    pos = find_col(ncol, rs, re, nA);
-                    if (pos >= 0) {
+#pragma unroll
+                for (int l = 0; l < NSD; ++l) {
+                    double s = 0;
+#pragma unroll
+                    for (int d = 0; d < NSD; ++d) s += prm.Uhat[d] * inv[l][d];
+                    *c++ = s;
+                }
+            }
+        }
+        if (pre) next = __ldg(off + next);
+        __syncwarp();
+        if (want_R)
+            for (int A = lane; A < nen; A += 32) {
+                double R = 0;
+#pragma unroll 3
+                for (int q = 0; q < nq; ++q) {
+                    const double NA = __ldg(tN + q * nen + A), w = coef[q * CO];
+                    if (PHYS == YG_SUPG) {
+                        double s = NSD * NA * prm.p[3];
+#pragma unroll
+                        for (int l = 0; l < NSD; ++l) s += coef[q * CO + 1 + NSD * NSD + NSD + l] * T[l * plane + q * S + (q >> 2) + A];
+                        R -= s * w;
+                    } else {
+                        R += NA * w;
+                    }
+                }
+                // one cell per launch adds to a node (or one lists it twice)
+#pragma unroll
+                for (int comp = 0; comp < DPN; ++comp)
+                    atomicAdd(residual + (int64_t)ge[3 * A] * DPN + comp,
+                              PHYS == YG_SUPG ? R : prm.p[(PHYS == YG_POISSON ? 1 : 3) + comp] * R);
+            }
+        if (pre) n = __ldg(el + next + lane);
+        for (int tl = 0; want_K && tl < ntiles; ++tl) {
+            int ta, tb;
+            if (SYM) {  // row-major over the upper triangle of tiles
+                ta = 0;
+                int rem = tl;
+                while (rem >= nt - ta) { rem -= nt - ta; ++ta; }
+                tb = ta + rem;
+            } else {
+                ta = tl / nt;
+                tb = tl - ta * nt;
+            }
+            const bool both = SYM && ta != tb;
+            // where node pair (A, B), A the row, lies: its position with bit 31 clear
+            // when it is stored, set when it is added to; -1 when there is none
+            auto position = [&](int A, int B) -> int {
+                if (A >= nen || B >= nen) return -1;
+                if (cmap) {
+                    const int m = __ldg(cmap + A * nen + B);
+                    return (ge[3 * A + 1] + (m & 0x7fff)) | (m & 0x8000 ? 0 : (int)0x80000000);
+                }
+                const int k = find_col(ncol, ge[3 * A + 1], ge[3 * A + 1] + ge[3 * A + 2], ge[3 * B]);
+                return k < 0 ? -1 : (k | (int)0x80000000);
+            };
+            const int ra = lane >> 2, rb = 2 * (lane & 3);  // lane's rows and columns of a fragment
+            // a tile's pairs are scattered row by row (8 r + c), but column by column
+            // where it has fewer columns than rows, so that the pairs there are come first
+            const int na = min(8, nen - 8 * ta), nb = min(8, nen - 8 * tb);
+            const bool by_col = nb < na;
+            // E == 1: pos[2 * f + h], the lane's own two pairs; else pos[2 * f + half],
+            // pair 32 half + lane of the order above
+            int pos[4];
+#pragma unroll
+            for (int f = 0; f < 2; ++f)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int hi = 4 * h + (lane >> 3), lo = lane & 7;
+                    const int a = E == 1 ? (f ? rb + h : ra) : (f || !by_col ? hi : lo);
+                    const int b = E == 1 ? (f ? ra : rb + h) : (f || !by_col ? lo : hi);
+                    pos[2 * f + h] = f && !both ? -1 : position(8 * (f ? tb : ta) + a, 8 * (f ? ta : tb) + b);
+                }
+            double C[NC][2];
+#pragma unroll
+            for (int i = 0; i < NC; ++i) C[i][0] = C[i][1] = 0;
+            // fragments: lane l holds point l % 4 and node l / 4 (clamped: entries past nen are dropped)
+            const double *Ta = T + (lane & 3) * S + min(8 * ta + ra, nen - 1);
+            const double *Tb = T + (lane & 3) * S + min(8 * tb + ra, nen - 1);
+            const double2 *cq = reinterpret_cast<const double2 *>(coef + (lane & 3) * CO);
+            for (int q0 = 0; q0 < nqp; q0 += 4, Ta += 4 * S + 1, Tb += 4 * S + 1, cq += 2 * CO) {
+                double da[NSD], db[NSD], c[CO];
+#pragma unroll
+                for (int j = 0; j < NSD; ++j) {
+                    da[j] = Ta[j * plane];
+                    db[j] = Tb[j * plane];
+                }
+#pragma unroll
+                for (int k = 0; k < (PHYS == YG_SUPG ? 1 + NSD * NSD + NSD + 1 : CO) / 2; ++k) {
+                    const double2 v = cq[k];
+                    c[2 * k] = v.x;
+                    c[2 * k + 1] = v.y;
+                }
+                if (PHYS == YG_ELASTICITY) {
+                    double b[NSD];
+#pragma unroll
+                    for (int d = 0; d < NSD; ++d) {
+                        b[d] = 0;
+#pragma unroll
+                        for (int j = 0; j < NSD; ++j) b[d] += c[1 + j * NSD + d] * db[j];
+                    }
+#pragma unroll
+                    for (int i = 0; i < NSD; ++i) {
+                        double a = 0;
+#pragma unroll
+                        for (int j = 0; j < NSD; ++j) a += c[1 + j * NSD + i] * da[j];
+                        a *= c[0];
+#pragma unroll
+                        for (int k = 0; k < NSD; ++k) dmma8x8x4(C[(i * NSD + k) % NC], a, b[k]);
+                    }
+                } else {
+                    const double NA = PHYS == YG_SUPG && q0 + (lane & 3) < nq
+                                          ? __ldg(tN + (q0 + (lane & 3)) * nen + min(8 * ta + ra, nen - 1)) : 0.0;
+#pragma unroll
+                    for (int l = 0; l < NSD; ++l) {
+                        double s = 0;
+#pragma unroll
+                        for (int j = 0; j < NSD; ++j) {
+                            const int lo = j < l ? j : l, hi = j < l ? l : j;
+                            s += da[j] * c[PHYS == YG_SUPG ? 1 + j * NSD + l : 1 + lo * NSD - lo * (lo - 1) / 2 + hi - lo];
+                        }
+                        if (PHYS == YG_SUPG) s += NA * c[1 + NSD * NSD + l];
+                        dmma8x8x4(C[0], s, db[l]);
+                    }
+                }
+            }
+            if (PHYS == YG_ELASTICITY) {
+                const double sg = prm.p[0], lam = prm.p[1], mu = prm.p[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    double tr = 0;
+#pragma unroll
+                    for (int d = 0; d < NSD; ++d) tr += C[d * NSD + d][h];
+#pragma unroll
+                    for (int i = 0; i < NSD; ++i) {
+                        C[i * NSD + i][h] = sg * (lam * C[i * NSD + i][h] + mu * (tr + C[i * NSD + i][h]));
+#pragma unroll
+                        for (int k = i + 1; k < NSD; ++k) {
+                            const double u = C[i * NSD + k][h], v = C[k * NSD + i][h];
+                            C[i * NSD + k][h] = sg * (lam * u + mu * v);
+                            C[k * NSD + i][h] = sg * (lam * v + mu * u);
+                        }
+                    }
+                }
+            } else if (PHYS == YG_POISSON) {
+                C[0][0] *= prm.p[0];
+                C[0][1] *= prm.p[0];
+            }
+            if (E == 1) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (pos[k] != -1) {
+                        double *v = val + (pos[k] & 0x7fffffff);
+                        if (pos[k] >= 0) *v = C[0][k & 1];
+                        else atomicAdd(v, C[0][k & 1]);
+                    }
+            } else {
+                constexpr int PP = 32 / E;  // blocks per step
+                const int sub = lane / E, e = lane - sub * E;
+                for (int f = 0; f < (both ? 2 : 1); ++f) {
+                    const int pairs = 8 * (f || by_col ? nb : na);
+                    // f = 0: rows A; f = 1: the transpose, rows B.  Pair p lies at p E + p / 16:
+                    // the four rows of a half warp's stores then use different banks
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int pair = f || by_col ? (rb + h) * 8 + ra : ra * 8 + rb + h;
+                        double *o = tile + pair * E + (pair >> 4);
 #pragma unroll
                         for (int i = 0; i < DPN; ++i)
 #pragma unroll
-                            for (int k = 0; k < DPN; ++k) val[entry_addr(format, DPN, nrp, nB, pos, k, i)] += K[i][k];
+                            for (int k = 0; k < DPN; ++k)
+                                o[i * DPN + k] = f ? C[(k * DPN + i) % NC][h] : C[(i * DPN + k) % NC][h];
                     }
-                }
-            }
-        }
-        if (want_R) {
-            for (int a = threadIdx.x; a < nen * DPN; a += blockDim.x) {
-                const int A = a / DPN, comp = a % DPN;
-                double R = 0;
-                for (int q = 0; q < nq; ++q) {
-                    const double NA = tN[(size_t)q * nen + A];
-                    if (PHYS == YG_POISSON) {
-                        R += (prm.p[1] * jxw[q]) * NA;
-                    } else if (PHYS == YG_ELASTICITY) {
-                        R += prm.p[3 + comp] * NA * jxw[q];
-                    } else {
-                        const double *gA = G + ((size_t)q * nen + A) * NSD;
+                    __syncwarp();
 #pragma unroll
-                        for (int ac = 0; ac < NSD; ++ac) R -= (NA * prm.p[3] + prm.Uhat[ac] * gA[ac]) * jxw[q];
+                    for (int half = 0; half < 2; ++half) {
+                        const int mine = f ? pos[2 + half] : pos[half];
+#pragma unroll
+                        for (int u = 0; u < (32 + PP - 1) / PP; ++u) {
+                            if (32 * half + PP * u >= pairs) break;
+                            const int pair = PP * u + sub;
+                            const int where = __shfl_sync(0xffffffffu, mine, pair & 31);
+                            const bool on = where != -1 && sub < PP && pair < 32;
+                            const double v = tile[min(32 * half + pair, 63) * E + min(2 * half + (pair >> 4), 3) + e];
+                            double *o = val + (int64_t)(where & 0x7fffffff) * E + e;
+                            if (!BCSR && on) {  // scalar rows of the node row
+                                const int A = f ? 8 * tb + 4 * half + (pair >> 3)
+                                                : 8 * ta + (by_col ? pair & 7 : 4 * half + (pair >> 3));
+                                const int rs = ge[3 * A + 1];
+                                o = val + (int64_t)rs * E + (int64_t)(e / DPN) * ge[3 * A + 2] * DPN +
+                                    (int64_t)((where & 0x7fffffff) - rs) * DPN + e % DPN;
+                            }
+                            if (on && where >= 0) *o = v;
+                            if (on && where < 0) atomicAdd(o, v);
+                        }
                     }
+                    __syncwarp();  // the buffer is free again
                 }
-                residual[(int64_t)gn[A] * DPN + comp] += R;
             }
         }
-        __syncthreads();
+        if (pre) {
+            x = nodes[3 * (int64_t)n];
+            y = nodes[3 * (int64_t)n + 1];
+            z = nodes[3 * (int64_t)n + 2];
+            r0 = __ldg(nrp + n);
+            r1 = __ldg(nrp + n + 1);
+        }
+        __syncwarp();
     }
 }
 
+// The element sizes the library takes: shape gradients at every quadrature point
+// of one element within a block's shared memory (hexahedra p <= 3).
 static size_t assemble_smem(int nen, int nq, int nsd) {
     return sizeof(double) * (3 * nen + (size_t)nq * nen * nsd + nq + 9 * nq) + sizeof(int32_t) * nen + 16;
 }
 
-template <int NSD, int DPN, int PHYS>
+template <int NSD, int DPN, int PHYS, bool BCSR>
 static yg_status launch_assemble(yg_context ctx, const ElementGroup &g, yg_dofmap d, const PhysParams &prm, double *val,
-                                 int format, double *residual, int want_K, int want_R) {
+                                 double *residual, int want_K, int want_R) {
     const int nen = g.tab.nen, nq = g.tab.nq;
-    size_t smem = assemble_smem(nen, nq, NSD);
-    auto kern = k_assemble<NSD, DPN, PHYS>;
-    if (smem > ctx->smem_optin)
+    const size_t limit = assemble_smem(nen, nq, NSD);
+    if (limit > ctx->smem_optin)
         return fail(YG_UNSUPPORTED, "CGAssembly: element (nen %d, nq %d) needs %zu B of shared memory, the device "
-                    "allows %zu", nen, nq, smem, ctx->smem_optin);
-    if (smem > 48 * 1024) YG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                    "allows %zu", nen, nq, limit, ctx->smem_optin);
+    auto kern = k_assemble<NSD, DPN, PHYS, BCSR>;
+    auto smem_of = [&](int w) {
+        return sizeof(double) * ((size_t)asm_table_doubles(nen, nq, NSD) +
+                                 (size_t)w * asm_warp_doubles(nen, nq, NSD, DPN * DPN, PHYS));
+    };
+    YG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->smem_optin));
+    // warps per CTA: as many resident warps as the SM holds beside the CTAs' tables
+    int warps = 0, resident = 0;
+    for (int w = 1; w <= kAsmWarps; ++w) {
+        int per = 0;
+        if (smem_of(w) > ctx->smem_optin) break;
+        YG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 32 * w, smem_of(w)));
+        if (per * w >= warps * resident) { warps = w; resident = per; }
+    }
+    if (warps == 0 || resident == 0)
+        return fail(YG_UNSUPPORTED, "CGAssembly: element (nen %d, nq %d) needs %zu B of shared memory, the device "
+                    "allows %zu", nen, nq, smem_of(1), ctx->smem_optin);
     for (size_t c = 0; c + 1 < g.color_ptr.size(); ++c) {
-        int n = g.color_ptr[c + 1] - g.color_ptr[c];
+        const int first = g.color_ptr[c], n = g.color_ptr[c + 1] - first;
         if (n == 0) continue;
-        int grid = std::min(n, ctx->num_sms * 16);
-        kern<<<grid, 128, smem, ctx->stream>>>(g.d_order + g.color_ptr[c], n, d->d_offsets, d->d_elements, d->d_nodes,
-                                               g.d_tab, nen, nq, g.tab.dim, prm, d->d_nrowptr, d->d_ncol, val, format,
-                                               residual, want_K, want_R);
+        // at most one wave; a colour of few cells is spread over the SMs instead
+        const int w = std::max(1, std::min(warps, (n + ctx->num_sms - 1) / ctx->num_sms));
+        const int grid = std::min((n + w - 1) / w, ctx->num_sms * resident);
+        kern<<<grid, w * 32, smem_of(w), ctx->stream>>>(
+            g.d_order + first, n, g.d_map ? g.d_map + (size_t)first * nen * nen : nullptr, d->d_offsets, d->d_elements,
+            d->d_nodes, g.d_tab, nen, nq, prm, d->d_nrowptr, d->d_ncol, val, residual, want_K, want_R);
         YG_LAUNCHED(ctx);
     }
     YG_CUDA(cudaGetLastError());
@@ -467,10 +808,28 @@ static yg_status launch_assemble(yg_context ctx, const ElementGroup &g, yg_dofma
 template <int NSD>
 static yg_status dispatch_physics(yg_context ctx, const ElementGroup &g, yg_dofmap d, int kind, int dpn,
                                   const PhysParams &prm, double *val, int format, double *residual, int wK, int wR) {
-    if (kind == YG_POISSON && dpn == 1) return launch_assemble<NSD, 1, YG_POISSON>(ctx, g, d, prm, val, format, residual, wK, wR);
-    if (kind == YG_SUPG && dpn == 1) return launch_assemble<NSD, 1, YG_SUPG>(ctx, g, d, prm, val, format, residual, wK, wR);
-    if (kind == YG_ELASTICITY && dpn == NSD) return launch_assemble<NSD, NSD, YG_ELASTICITY>(ctx, g, d, prm, val, format, residual, wK, wR);
+    if (kind == YG_POISSON && dpn == 1) 
+        return launch_assemble<NSD, 1, YG_POISSON, true>(ctx, g, d, prm, val, residual, wK, wR);
+    if (kind == YG_SUPG && dpn == 1) 
+        return launch_assemble<NSD, 1, YG_SUPG, true>(ctx, g, d, prm, val, residual, wK, wR);
+    if (kind == YG_ELASTICITY && dpn == NSD) 
+        return format == YG_FORMAT_BCSR || NSD == 1
+                   ? launch_assemble<NSD, NSD, YG_ELASTICITY, true>(ctx, g, d, prm, val, residual, wK, wR)
+                   : launch_assemble<NSD, NSD, YG_ELASTICITY, NSD == 1>(ctx, g, d, prm, val, residual, wK, wR);
     return fail(YG_BAD_ARG, "physics %d needs dof_per_node %d (got %d)", kind, kind == YG_ELASTICITY ? NSD : 1, dpn);
+}
+
+// Frees the element groups (a scatter map is listed with the context while it lives).
+static void free_groups(yg_dofmap d) {
+    yg_context ctx = d->ctx;
+    for (auto &g : d->groups) {
+        dev_free(ctx, g.d_tab);
+        dev_free(ctx, g.d_order);
+        dev_free(ctx, g.d_map);
+        auto &o = ctx->optional;
+        o.erase(std::remove(o.begin(), o.end(), reinterpret_cast<void **>(&g.d_map)), o.end());
+    }
+    d->groups.clear();
 }
 
 // Node graph + element groups for simulation dimension nsd.
@@ -479,8 +838,7 @@ static yg_status build_pattern(yg_dofmap d, int nsd) {
     yg_context ctx = d->ctx;
     dev_free(ctx, d->d_nrowptr);
     dev_free(ctx, d->d_ncol);
-    for (auto &g : d->groups) { dev_free(ctx, g.d_tab); dev_free(ctx, g.d_order); }
-    d->groups.clear();
+    free_groups(d);
     d->d_nrowptr = d->d_ncol = nullptr;
     const HostDofmap &h = d->host;
     const int32_t nc = h.n_cells(), nn = h.n_nodes();
@@ -512,7 +870,11 @@ static yg_status build_pattern(yg_dofmap d, int nsd) {
     int8_t *d_inc = nullptr;
     int32_t *d_cnt = nullptr, *d_cursor = nullptr, *d_adj = nullptr, *d_rowcnt = nullptr, *d_flag = nullptr;
     int64_t *d_aptr = nullptr, *d_rp64 = nullptr;
+    ScatterMaps maps;
+    int32_t *d_slot = nullptr;
+    uint8_t *d_rank = nullptr;
     auto cleanup = [&]() {
+        dev_free(ctx, d_slot); dev_free(ctx, d_rank);
         dev_free(ctx, d_inc); dev_free(ctx, d_cnt); dev_free(ctx, d_cursor); dev_free(ctx, d_adj);
         dev_free(ctx, d_rowcnt); dev_free(ctx, d_flag); dev_free(ctx, d_aptr); dev_free(ctx, d_rp64);
     };
@@ -551,13 +913,48 @@ static yg_status build_pattern(yg_dofmap d, int nsd) {
     if (nnz >= INT32_MAX) { cleanup(); return fail(YG_UNSUPPORTED, "node graph too large for 32-bit offsets"); }
     TRYC(dev_alloc_t(ctx, &d->d_nrowptr, nn + 1));
     TRYC(dev_alloc_t(ctx, &d->d_ncol, nnz + 1));
+    // scatter maps: two bytes per element entry.  A context whose budget or
+    // memory does not hold them assembles without (k_assemble then searches).
+    bool mapped = nn > 0 && !d->groups.empty();
+    for (size_t g = 0; mapped && g < d->groups.size(); ++g) {
+        ElementGroup &gr = d->groups[g];
+        const size_t cells = gr.color_ptr.empty() ? 0 : (size_t)gr.color_ptr.back();
+        mapped = dev_alloc_t(ctx, &gr.d_map, cells * gr.tab.nen * gr.tab.nen) == YG_OK;
+        maps.map[g] = gr.d_map;
+        maps.nen[g] = gr.tab.nen;
+    }
+    mapped = mapped && dev_alloc_t(ctx, &d_slot, nc + 1) == YG_OK && dev_alloc_t(ctx, &d_rank, nc + 1) == YG_OK;
+    if (mapped) {
+        for (size_t g = 0; g < d->groups.size(); ++g) {
+            const ElementGroup &gr = d->groups[g];
+            for (size_t c = 0; c + 1 < gr.color_ptr.size(); ++c) {
+                const int first = gr.color_ptr[c], n = gr.color_ptr[c + 1] - first;
+                if (n == 0) continue;
+                k_cell_slots<<<stream_grid(ctx, n), kThreads, 0, st>>>(gr.d_order + first, n, first, (int)(64 * g + c),
+                                                                      d_slot, d_rank);
+                YG_LAUNCHED(ctx);
+            }
+        }
+        maps.slot = d_slot;
+        maps.rank = d_rank;
+    }
+    int32_t odd = 0;
     k_row_fill<<<rgrid, kRowWarps * 32, 0, st>>>(nn, d_aptr, d_adj, d->d_offsets, d->d_elements, d_rp64, d->d_nrowptr,
-                                                 d->d_ncol);
+                                                 d->d_ncol, maps, d_flag);
     YG_LAUNCHED(ctx);
+    cudaMemcpyAsync(&odd, d_flag, sizeof(int32_t), cudaMemcpyDeviceToHost, st);
     cudaError_t e = cudaStreamSynchronize(st);
     cleanup();
 #undef TRYC
     if (e != cudaSuccess) return fail(YG_CUDA_ERROR, "pattern build: %s", cudaGetErrorString(e));
+    for (auto &g : d->groups) {
+        if (mapped && !odd) {
+            ctx->optional.push_back(reinterpret_cast<void **>(&g.d_map));
+        } else {
+            dev_free(ctx, g.d_map);
+            g.d_map = nullptr;
+        }
+    }
     d->nnz_nodes = nnz;
     d->pattern_nsd = nsd;
     return YG_OK;
@@ -934,7 +1331,7 @@ extern "C" yg_status yg_dofmap_destroy(yg_dofmap d) {
     dev_free(ctx, d->d_elements);
     dev_free(ctx, d->d_nrowptr);
     dev_free(ctx, d->d_ncol);
-    for (auto &g : d->groups) { dev_free(ctx, g.d_tab); dev_free(ctx, g.d_order); }
+    free_groups(d);
     delete d;
     return YG_OK;
 }
@@ -987,7 +1384,11 @@ extern "C" yg_status yg_assemble(yg_dofmap d, const yg_physics *physics, uint32_
             return fail(YG_BAD_ARG, "matrix was not assembled from this dofmap in this format");
         }
         yg_matrix A = *K;
-        YG_CUDA(cudaMemsetAsync(A->d_val, 0, sizeof(double) * A->nnzb * A->block * A->block, ctx->stream));
+        // with scatter maps every entry is stored before it is added to
+        bool mapped = true;
+        for (const ElementGroup &g : d->groups) mapped = mapped && g.d_map;
+        if (!mapped || d->groups.empty())
+            YG_CUDA(cudaMemsetAsync(A->d_val, 0, sizeof(double) * A->nnzb * A->block * A->block, ctx->stream));
         val = A->d_val;
     }
     PhysParams prm{};

@@ -50,9 +50,21 @@ void flush_alloc_cache(yg_context ctx) {
     ctx->cached_bytes = 0;
 }
 
+// Frees the context's optional buffers; whether there were any.
+static bool release_optional(yg_context ctx) {
+    bool any = false;
+    for (void **p : ctx->optional) {
+        any = any || *p;
+        dev_free(ctx, *p);
+        *p = nullptr;
+    }
+    return any;
+}
+
 yg_status dev_alloc(yg_context ctx, void **p, size_t bytes) {
     *p = nullptr;
     if (bytes == 0) bytes = 16;
+    if (ctx->budget && ctx->in_use + bytes > ctx->budget) release_optional(ctx);
     if (ctx->budget && ctx->in_use + bytes > ctx->budget)
         return fail(YG_OVER_BUDGET, "allocation of %zu bytes exceeds the HBM budget (%llu of %llu in use)",
                     bytes, (unsigned long long)ctx->in_use, (unsigned long long)ctx->budget);
@@ -67,6 +79,11 @@ yg_status dev_alloc(yg_context ctx, void **p, size_t bytes) {
     } else {
         cudaError_t e = cudaMalloc(p, bytes);
         if (e != cudaSuccess && !ctx->cache.empty()) {  // give the cached blocks back and retry
+            cudaGetLastError();
+            flush_alloc_cache(ctx);
+            e = cudaMalloc(p, bytes);
+        }
+        if (e != cudaSuccess && release_optional(ctx)) {
             cudaGetLastError();
             flush_alloc_cache(ctx);
             e = cudaMalloc(p, bytes);

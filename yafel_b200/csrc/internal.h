@@ -76,6 +76,10 @@ struct yg_context_t {
     };
     std::multimap<size_t, CachedBlock> cache;
     size_t cached_bytes = 0;
+    // buffers that calls do without when memory is short (an assembly's scatter
+    // map): an allocation that would fail frees them all (the pointers become
+    // NULL) and tries again
+    std::vector<void **> optional;
     // reduction scratch (device) and pinned host mailbox
     double *d_partials = nullptr;   // 8 * kMaxReduceBlocks doubles
     double *h_pinned = nullptr;     // 64 doubles of pinned host memory
