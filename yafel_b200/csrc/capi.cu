@@ -322,7 +322,8 @@ extern "C" yg_status yg_context_create(int32_t device, uint64_t hbm_budget_bytes
     YG_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     yg_status s;
     if ((s = dev_alloc_t(ctx, &ctx->d_partials, 8 * kMaxReduceBlocks)) != YG_OK ||
-        (s = dev_alloc_t(ctx, &ctx->d_scalars, 4)) != YG_OK || (s = dev_alloc_t(ctx, &ctx->d_err, 4)) != YG_OK) {
+        (s = dev_alloc_t(ctx, &ctx->d_scalars, 4)) != YG_OK || (s = dev_alloc_t(ctx, &ctx->d_err, 4)) != YG_OK ||
+        (s = dev_alloc(ctx, &ctx->d_slots, 2 * 32 * 256)) != YG_OK) {
         yg_context_destroy(ctx);
         return s;
     }

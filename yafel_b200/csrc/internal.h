@@ -85,6 +85,7 @@ struct yg_context_t {
     double *h_pinned = nullptr;     // 64 doubles of pinned host memory
     KrylovScalars *d_scalars = nullptr;
     int32_t *d_err = nullptr;       // device-side error word (bounded waits that expired)
+    void *d_slots = nullptr;        // grid-wide sums of the cooperative kernels: 2 x 32 bytes per block, 256 blocks
     int reduce_blocks = 592;        // persistent grid for fused Krylov kernels
 };
 
@@ -184,6 +185,13 @@ yg_status vector_dot(yg_context ctx, const double *a, const double *b, int64_t n
 yg_status check_device_error(yg_context ctx);
 yg_status matrix_build_diag(yg_matrix A);
 void flush_alloc_cache(yg_context ctx);
+// Smallest and largest row length of A into row_min / row_max, measured once.
+yg_status matrix_row_extent(yg_matrix A);
+// PCG iterations in one cooperative kernel (pcg_resident.cu)
+yg_status launch_cooperative(yg_context ctx, const void *kern, int grid, int threads, size_t smem, void **args);
+yg_status pcg_resident_fits(yg_matrix A, bool f32, bool jacobi, bool *fits);
+yg_status pcg_resident_launch(yg_matrix A, bool f32, const double *dinv, double *x, double *r, double *p, double *zp,
+                              int max_its, int check, double rr_replace);
 // batch engine, host side (batch.cu)
 bool batch_slot_running(yg_batch bt, int32_t slot);
 void batch_slot_stats(yg_batch bt, int32_t slot, yg_solve_stats *out);

@@ -13,7 +13,8 @@
 // iteration parity so no block reads a value another block of the same kernel
 // is writing.  A run of iterations is captured once into a CUDA graph and
 // replayed; kernels return immediately once the flag is set, and the host reads
-// the flag once per replay.  All reductions have a fixed order, so a solve is
+// the flag once per replay.  Systems whose matrix fits the shared memory of the SMs
+// run the same iteration in one cooperative kernel instead (pcg_resident.cu).  All reductions have a fixed order, so a solve is
 // bit-reproducible.  ILU(0) goes through the general path (z stored, apply by
 // precond.cu, then a separate r.z reduction).
 #include "internal.h"
@@ -286,10 +287,10 @@ struct Work {
     yg_context ctx;
     int64_t n;
     double *r = nullptr, *p = nullptr, *q = nullptr, *z = nullptr, *t = nullptr, *s = nullptr, *v = nullptr,
-           *rhat = nullptr, *ph = nullptr, *sh = nullptr, *d = nullptr;
+           *rhat = nullptr, *ph = nullptr, *sh = nullptr, *d = nullptr, *zp = nullptr;  // zp: resident iterations only
     Dir32 d32;  // FP32 copy of p for the mixed-precision SpMV (p32 NULL otherwise)
     ~Work() {
-        for (double *ptr : {r, p, q, z, t, s, v, rhat, ph, sh, d}) dev_free(ctx, ptr);
+        for (double *ptr : {r, p, q, z, t, s, v, rhat, ph, sh, d, zp}) dev_free(ctx, ptr);
         dev_free(ctx, d32.p32);
     }
 };
@@ -484,14 +485,20 @@ static yg_status pcg_core(yg_matrix A, yg_precond M, const double *b, double *x,
     if (hs.flag == FLAG_RUN || (hs.flag == FLAG_CONVERGED && criterion == YG_CRIT_RELRES && hs.iter > 0)) {
         IterGraph g;
         if (prof && prof->on && prof->start.empty()) YG_TRY(prof->init(check_every));
-        YG_TRY(capture(ctx, check_every, one, g));
+        if (!w.zp) YG_TRY(capture(ctx, check_every, one, g));
         double rr_last = hs.rr;  // r.r at the last replacement
         int false_stops = 0;
         for (;;) {
             int64_t before = hs.iter;
-            YG_CUDA(cudaGraphLaunch(g.exec, st));
-            ctx->launches += g.kernels;
+            if (w.zp) {
+                YG_TRY(pcg_resident_launch(A, f32, dinv, x, w.r, w.p, w.zp, 1 << 12, check_every,
+                                           reliable ? 1e-2 * rr_last : 0.0));
+            } else {
+                YG_CUDA(cudaGraphLaunch(g.exec, st));
+                ctx->launches += g.kernels;
+            }
             YG_TRY(read_scalars(ctx, &hs));
+            if (w.zp && hs.flag == FLAG_NAN) YG_TRY(check_device_error(ctx));  // or a grid-wide sum that timed out
             if (prof) YG_TRY(prof->collect(hs.iter - before));
             if (hs.flag == FLAG_RUN) {
                 // replace once the recursive residual fell 10x since the last time
@@ -543,7 +550,15 @@ yg_status solve_cg(yg_matrix A, yg_precond M, yg_vector bv, yg_vector xv, const 
     YG_TRY(alloc_vec(ctx, &w.p, n));
     YG_TRY(alloc_vec(ctx, &w.q, n));
     if (M && !precond_fusable(M)) YG_TRY(alloc_vec(ctx, &w.z, n));
-    if (o.precision != YG_PREC_FP64 && (A->block == 2 || A->block == 3)) {
+    if (o.precision != YG_PREC_FP64 && !A->d_val32) YG_TRY(yg_matrix_make_fp32(A));
+    // Systems whose matrix fits the SMs' shared memory iterate there; the others
+    // stream it through the SpMV kernel that suits them best.
+    bool resident = false;
+    if (precond_fusable(M) && !o.profile)
+        YG_TRY(pcg_resident_fits(A, o.precision != YG_PREC_FP64, precond_dinv(M) != nullptr, &resident));
+    if (resident && alloc_vec(ctx, &w.zp, 2 * n) != YG_OK) resident = false;  // no room beside the budget
+    if (!resident) YG_TRY(spmv_autotune_device(A));  // the FP32-value kernel has its own tuning
+    if (!resident && o.precision != YG_PREC_FP64 && (A->block == 2 || A->block == 3)) {
         // FP32 gather copy of p (node-padded) for the FP32-value TMA SpMV
         const int xs = spmv_x32_stride(A->block);
         const int64_t m32 = (n / A->block + 1) * xs;
@@ -564,8 +579,6 @@ yg_status solve_cg(yg_matrix A, yg_precond M, yg_vector bv, yg_vector xv, const 
     if (o.precision == YG_PREC_FP64 || o.precision == YG_PREC_MIXED) {
         // FP64, or FP32 matrix values in the iteration with the residual replaced
         // by the FP64 true residual each time it fell 10x (refinement steps).
-        if (o.precision == YG_PREC_MIXED && !A->d_val32) YG_TRY(yg_matrix_make_fp32(A));
-        YG_TRY(spmv_autotune_device(A));  // the FP32-value kernel has its own tuning
         int64_t repl = 0;
         YG_TRY(pcg_core(A, M, bv->d, xv->d, o.precision, o.criterion, o.tol, maxiter, m, w, &its, &flag, &prof,
                         &repl));
@@ -575,8 +588,6 @@ yg_status solve_cg(yg_matrix A, yg_precond M, yg_vector bv, yg_vector xv, const 
         // YG_PREC_MIXED_IR: restarted FP64 iterative refinement around a PCG whose
         // SpMV reads FP32 values (FP64 vectors and accumulation).  Outer residuals
         // and the final check are FP64.
-        if (!A->d_val32) YG_TRY(yg_matrix_make_fp32(A));
-        YG_TRY(spmv_autotune_device(A));
         YG_TRY(alloc_vec(ctx, &w.d, n));
         YG_TRY(alloc_vec(ctx, &w.t, n));
         double bnorm = 0;
@@ -641,7 +652,6 @@ extern "C" yg_status yg_cg(yg_matrix A, yg_precond M, yg_vector b, yg_vector x, 
     if (opts && opts->precision != YG_PREC_FP64 && opts->precision != YG_PREC_MIXED &&
         opts->precision != YG_PREC_MIXED_IR)
         return fail(YG_BAD_ARG, "yg_cg: precision %d is not a solver precision", (int)opts->precision);
-    YG_TRY(spmv_autotune_device(A));
     yg_status s = solve_cg(A, M, b, x, opts, stats);
     if (s != YG_OK && s != YG_NOT_CONVERGED && s != YG_BREAKDOWN && s != YG_NAN) return s;
     if (s != YG_OK) set_error("yg_cg: %s", yg_status_string(s));

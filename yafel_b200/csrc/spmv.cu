@@ -793,7 +793,7 @@ __global__ void k_row_tiles(int64_t n, int64_t nt, int64_t per, const int32_t *_
 }
 
 // Smallest and largest number of entries (blocks) per row of A, measured once.
-static yg_status row_extent(yg_matrix A) {
+yg_status matrix_row_extent(yg_matrix A) {
     if (A->row_min >= 0) return YG_OK;
     yg_context ctx = A->ctx;
     cudaStreamCaptureStatus cs;
@@ -826,7 +826,7 @@ static yg_status csr_tiles_build(yg_matrix A, int k) {
     cudaStreamCaptureStatus cs;
     YG_CUDA(cudaStreamIsCapturing(ctx->stream, &cs));
     if (cs != cudaStreamCaptureStatusNone) return fail(YG_BAD_ARG, "row tiles cannot be built during stream capture");
-    YG_TRY(row_extent(A));
+    YG_TRY(matrix_row_extent(A));
     const int cap = 256 << k;
     if (A->row_min < 1 || A->row_max > cap)
         return fail(YG_UNSUPPORTED, "row-tile SpMV needs 1..%d entries per row (rows hold %d..%d)", cap, A->row_min,
@@ -850,7 +850,7 @@ yg_status spmv_prepare(yg_matrix A, int variant, int lanes) {
             return fail(YG_BAD_ARG, "whole-row SpMV configurations are lanes 1, 2, 4, 8");
         if (A->block != 2 && A->block != 3) return fail(YG_UNSUPPORTED, "whole-row SpMV needs 2x2 or 3x3 blocks");
         if (A->nbrows >= INT32_MAX) return fail(YG_UNSUPPORTED, "whole-row SpMV needs fewer than 2^31 block rows");
-        YG_TRY(row_extent(A));
+        YG_TRY(matrix_row_extent(A));
         if (A->row_max > rows_capacity_of(lanes))
             return fail(YG_UNSUPPORTED, "whole-row SpMV (lanes %d) holds rows of up to %d blocks; the longest has %d",
                         lanes, rows_capacity_of(lanes), A->row_max);
