@@ -47,6 +47,9 @@ struct ElementGroup {
     // entry's position in its node row, bit 15 set when no earlier cell (group, then
     // colour) touches it; NULL when it could not be built (see build_pattern)
     uint16_t *d_map = nullptr;
+    // launch shape of the last assembly kernel run on the group (warps per CTA, CTAs per SM)
+    mutable const void *shaped = nullptr;
+    mutable int warps = 0, resident = 0;
 };
 
 struct yg_dofmap_t {
@@ -203,11 +206,17 @@ k_row_count(int32_t nnodes, const int64_t *__restrict__ aptr, const int32_t *__r
 
 // Where the cells of an assembly group stand: position in the group's colour
 // order and rank (64 * group + colour), by which cells of one node are told apart.
-__global__ void k_cell_slots(const int32_t *__restrict__ order, int n, int first, int rank, int32_t *__restrict__ slot,
-                             uint8_t *__restrict__ ranks) {
+struct ColorPtr {
+    int32_t at[65];  // first position of each colour, then the end
+};
+__global__ void k_cell_slots(const int32_t *__restrict__ order, ColorPtr color, int ncolors, int group,
+                             int32_t *__restrict__ slot, uint8_t *__restrict__ ranks) {
+    const int n = color.at[ncolors];
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        slot[order[t]] = first + t;
-        ranks[order[t]] = (uint8_t)rank;
+        int c = 0;
+        while (color.at[c + 1] <= t) ++c;
+        slot[order[t]] = t;
+        ranks[order[t]] = (uint8_t)(64 * group + c);
     }
 }
 
@@ -393,7 +402,7 @@ constexpr int kAsmWarps = 10;  // warps per CTA at most
 // Values alone (tangent; all colours), against a CTA per cell that formed every
 // entry by vector FMAs and read, added and wrote back the cleared values:
 // 33^3 Q2 hexahedra 3x3 blocks 2.81 -> 1.39 ms, 48^3 Q1 1.24 -> 0.41 ms, 14^3 Q3 5.29 ->
-// 1.82 ms, scalar 37^3 Q2 2.23 -> 0.71 ms, 60^3 Q1 1.53 -> 0.25 ms, 200^2 Q2 2x2 blocks
+// 0.84 ms, scalar 37^3 Q2 2.23 -> 0.71 ms, 60^3 Q1 1.53 -> 0.25 ms, 200^2 Q2 2x2 blocks
 // 0.33 -> 0.13 ms.  Floors of the first: 161k FMA per cell, 0.16 ms at the 37
 // TFLOP/s the matrix instructions reach; 26.2M block updates of 72 bytes, 18.6M of
 // them first touches, 0.37 ms.  What bounds it now is the shared-memory pipe (65 %
@@ -405,7 +414,7 @@ k_assemble(const int32_t *__restrict__ order, int ncell, const uint16_t *__restr
            const int32_t *__restrict__ off, const int32_t *__restrict__ el, const double *__restrict__ nodes,
            const double *__restrict__ tab, int nen, int nq, PhysParams prm, const int32_t *__restrict__ nrp,
            const int32_t *__restrict__ ncol, double *__restrict__ val, double *__restrict__ residual, int want_K,
-           int want_R) {
+           int want_R, int split) {
     extern __shared__ __align__(16) double sm[];
     constexpr bool SYM = (PHYS != YG_SUPG);
     constexpr int NC = PHYS == YG_ELASTICITY ? NSD * NSD : 1;  // accumulators per tile
@@ -432,15 +441,16 @@ k_assemble(const int32_t *__restrict__ order, int ncell, const uint16_t *__restr
     // the lane's node of the next cell, fetched a cell ahead, one dependent load per step
     int n = 0, r0 = 0, r1 = 0;
     double x = 0, y = 0, z = 0;
-    if (t < ncell && lane < nen) {
-        n = el[off[order[t]] + lane];
+    if (t / split < ncell && lane < nen) {
+        n = el[off[order[t / split]] + lane];
         r0 = nrp[n];
         r1 = nrp[n + 1];
         x = nodes[3 * (int64_t)n];
         y = nodes[3 * (int64_t)n + 1];
         z = nodes[3 * (int64_t)n + 2];
     }
-    for (; t < ncell; t += nteams) {
+    for (; t / split < ncell; t += nteams) {
+        const int cell = t / split, part = t - cell * split;
         auto put_node = [&](int a) {
             xe[3 * a] = x;
             xe[3 * a + 1] = y;
@@ -451,7 +461,7 @@ k_assemble(const int32_t *__restrict__ order, int ncell, const uint16_t *__restr
         };
         if (lane < nen) put_node(lane);
         if (nen > 32) {
-            const int base = off[order[t]];
+            const int base = off[order[cell]];
             for (int a = lane + 32; a < nen; a += 32) {
                 n = el[base + a];
                 r0 = nrp[n];
@@ -462,12 +472,12 @@ k_assemble(const int32_t *__restrict__ order, int ncell, const uint16_t *__restr
                 put_node(a);
             }
         }
-        const uint16_t *cmap = map ? map + (int64_t)t * nen * nen : nullptr;
+        const uint16_t *cmap = map ? map + (int64_t)cell * nen * nen : nullptr;
         if (map && want_K)
             for (int i = 64 * lane; i < nen * nen; i += 64 * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(cmap + i));
-        const bool pre = t + nteams < ncell && lane < nen;
+        const bool pre = (t + nteams) / split < ncell && lane < nen;
         int next = 0;
-        if (pre) next = __ldg(order + t + nteams);
+        if (pre) next = __ldg(order + (t + nteams) / split);
         __syncwarp();
         // Element::update, a lane per quadrature point: Jacobian, det, inverse
         for (int q = lane; q < nq; q += 32) {
@@ -559,7 +569,7 @@ k_assemble(const int32_t *__restrict__ order, int ncell, const uint16_t *__restr
         }
         if (pre) next = __ldg(off + next);
         __syncwarp();
-        if (want_R)
+        if (want_R && part == 0)
             for (int A = lane; A < nen; A += 32) {
                 double R = 0;
 #pragma unroll 3
@@ -581,7 +591,7 @@ k_assemble(const int32_t *__restrict__ order, int ncell, const uint16_t *__restr
                               PHYS == YG_SUPG ? R : prm.p[(PHYS == YG_POISSON ? 1 : 3) + comp] * R);
             }
         if (pre) n = __ldg(el + next + lane);
-        for (int tl = 0; want_K && tl < ntiles; ++tl) {
+        for (int tl = part; want_K && tl < ntiles; tl += split) {
             int ta, tb;
             if (SYM) {  // row-major over the upper triangle of tiles
                 ta = 0;
@@ -778,27 +788,36 @@ static yg_status launch_assemble(yg_context ctx, const ElementGroup &g, yg_dofma
         return sizeof(double) * ((size_t)asm_table_doubles(nen, nq, NSD) +
                                  (size_t)w * asm_warp_doubles(nen, nq, NSD, DPN * DPN, PHYS));
     };
-    YG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->smem_optin));
-    // warps per CTA: as many resident warps as the SM holds beside the CTAs' tables
-    int warps = 0, resident = 0;
-    for (int w = 1; w <= kAsmWarps; ++w) {
-        int per = 0;
-        if (smem_of(w) > ctx->smem_optin) break;
-        YG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 32 * w, smem_of(w)));
-        if (per * w >= warps * resident) { warps = w; resident = per; }
+    if (g.shaped != reinterpret_cast<const void *>(kern)) {
+        YG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->smem_optin));
+        // warps per CTA: as many resident warps as the SM holds beside the CTAs' tables
+        g.warps = g.resident = 0;
+        for (int w = 1; w <= kAsmWarps; ++w) {
+            int per = 0;
+            if (smem_of(w) > ctx->smem_optin) break;
+            YG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 32 * w, smem_of(w)));
+            if (per * w >= g.warps * g.resident) { g.warps = w; g.resident = per; }
+        }
+        if (g.warps == 0 || g.resident == 0)
+            return fail(YG_UNSUPPORTED, "CGAssembly: element (nen %d, nq %d) needs %zu B of shared memory, the device "
+                        "allows %zu", nen, nq, smem_of(1), ctx->smem_optin);
+        g.shaped = reinterpret_cast<const void *>(kern);
     }
-    if (warps == 0 || resident == 0)
-        return fail(YG_UNSUPPORTED, "CGAssembly: element (nen %d, nq %d) needs %zu B of shared memory, the device "
-                    "allows %zu", nen, nq, smem_of(1), ctx->smem_optin);
+    const int warps = g.warps, resident = g.resident;
     for (size_t c = 0; c + 1 < g.color_ptr.size(); ++c) {
         const int first = g.color_ptr[c], n = g.color_ptr[c + 1] - first;
         if (n == 0) continue;
-        // at most one wave; a colour of few cells is spread over the SMs instead
-        const int w = std::max(1, std::min(warps, (n + ctx->num_sms - 1) / ctx->num_sms));
-        const int grid = std::min((n + w - 1) / w, ctx->num_sms * resident);
+        // at most one wave.  A colour of fewer cells than warps is spread over the SMs,
+        // and its cells over `split` warps that each form a share of the tiles (12^3 Q2
+        // hexahedra, 216 cells a colour: 0.36 ms with a warp per cell, 0.16 with ten)
+        const int nt = (nen + 7) / 8, tiles = PHYS == YG_SUPG ? nt * nt : nt * (nt + 1) / 2;
+        const int split = want_K ? std::max(1, std::min(tiles, ctx->num_sms * resident * warps / n)) : 1;
+        const int64_t teams = (int64_t)n * split;
+        const int w = (int)std::max<int64_t>(1, std::min<int64_t>(warps, (teams + ctx->num_sms - 1) / ctx->num_sms));
+        const int grid = (int)std::min<int64_t>((teams + w - 1) / w, (int64_t)ctx->num_sms * resident);
         kern<<<grid, w * 32, smem_of(w), ctx->stream>>>(
             g.d_order + first, n, g.d_map ? g.d_map + (size_t)first * nen * nen : nullptr, d->d_offsets, d->d_elements,
-            d->d_nodes, g.d_tab, nen, nq, prm, d->d_nrowptr, d->d_ncol, val, residual, want_K, want_R);
+            d->d_nodes, g.d_tab, nen, nq, prm, d->d_nrowptr, d->d_ncol, val, residual, want_K, want_R, split);
         YG_LAUNCHED(ctx);
     }
     YG_CUDA(cudaGetLastError());
@@ -927,11 +946,12 @@ static yg_status build_pattern(yg_dofmap d, int nsd) {
     if (mapped) {
         for (size_t g = 0; g < d->groups.size(); ++g) {
             const ElementGroup &gr = d->groups[g];
-            for (size_t c = 0; c + 1 < gr.color_ptr.size(); ++c) {
-                const int first = gr.color_ptr[c], n = gr.color_ptr[c + 1] - first;
-                if (n == 0) continue;
-                k_cell_slots<<<stream_grid(ctx, n), kThreads, 0, st>>>(gr.d_order + first, n, first, (int)(64 * g + c),
-                                                                      d_slot, d_rank);
+            ColorPtr color;
+            const int nc_ = (int)gr.color_ptr.size() - 1;
+            for (int c = 0; c <= nc_; ++c) color.at[c] = gr.color_ptr[c];
+            if (nc_ > 0 && gr.color_ptr[nc_] > 0) {
+                k_cell_slots<<<stream_grid(ctx, gr.color_ptr[nc_]), kThreads, 0, st>>>(gr.d_order, color, nc_, (int)g, d_slot,
+                                                                                      d_rank);
                 YG_LAUNCHED(ctx);
             }
         }
