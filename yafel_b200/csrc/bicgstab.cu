@@ -25,7 +25,6 @@ namespace yg {
 int stream_grid(yg_context ctx, int64_t n);
 bool precond_fusable(yg_precond M);
 const double *precond_dinv(yg_precond M);
-yg_status precond_apply_dev(yg_precond M, const double *r, double *z);
 
 enum { BF_RUN = 0, BF_CONVERGED = 1, BF_BREAKDOWN = 2, BF_NAN = 3, BF_MAXITER = 4 };
 

@@ -139,14 +139,12 @@ struct yg_precond_t {
     int32_t kind = 0;
     double *d_dinv = nullptr;     // Jacobi: 1/a_ii (scalar diagonal)
     int64_t zero_pivots = 0;
-    // ILU(0): factor values on A's pattern (scalar CSR view) + level schedules
+    // ILU(0): factor values on A's pattern (scalar rows of a block row one after the
+    // other), block rows sorted by dependency level, the two vectors an apply polls
     double *d_lu = nullptr;
-    int32_t *d_lower_levels = nullptr, *d_upper_levels = nullptr;  // row lists grouped by level
-    std::vector<int32_t> lower_level_ptr, upper_level_ptr;
-    int32_t *d_csr_rowptr = nullptr, *d_csr_col = nullptr, *d_csr_diag = nullptr;  // scalar view
-    int32_t *d_lower_ptr = nullptr, *d_upper_ptr = nullptr;  // level pointers for the persistent sweeps
-    uint32_t *d_bar = nullptr;                              // their grid barrier (count, generation)
-    int64_t n = 0, nnz = 0;
+    int32_t *d_lower_rows = nullptr, *d_upper_rows = nullptr;
+    double *d_z = nullptr;
+    int64_t lower_levels = 0, upper_levels = 0;  // of the scalar rows
     double *d_tmp = nullptr;
 };
 

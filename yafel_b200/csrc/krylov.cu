@@ -26,7 +26,7 @@
 
 namespace yg {
 
-yg_status precond_apply_dev(yg_precond M, const double *r, double *z);
+yg_status precond_apply_dev(yg_precond M, const double *r, double *z, const int32_t *flag = nullptr);
 bool precond_fusable(yg_precond M);
 const double *precond_dinv(yg_precond M);
 int stream_grid(yg_context ctx, int64_t n);
@@ -450,7 +450,7 @@ static yg_status pcg_core(yg_matrix A, yg_precond M, const double *b, double *x,
         } else {
             k_cg_update<false><<<G, kThreads, 0, st>>>(n, P, spmv_grid, S, parity, x, w.r, w.p, w.q, nullptr, P + 2 * G);
             YG_LAUNCHED(ctx);
-            YG_TRY(precond_apply_dev(M, w.r, w.z));
+            YG_TRY(precond_apply_dev(M, w.r, w.z, &S->flag));
             k_dot2_partials<<<G, kThreads, 0, st>>>(n, w.r, w.z, P + 2 * G, &S->flag, 0, 2);
             YG_LAUNCHED(ctx);
             k_cg_pupdate<false><<<G, kThreads, 0, st>>>(n, P + 2 * G, G, S, parity, w.p, w.r, w.z, nullptr, d32);

@@ -325,6 +325,13 @@ yg_status launch_cooperative(yg_context ctx, const void *kern, int grid, int thr
     static std::mutex m;
     static cudaEvent_t last[64] = {};
     const int d = ctx->device & 63;
+    cudaStreamCaptureStatus cs;
+    YG_CUDA(cudaStreamIsCapturing(ctx->stream, &cs));
+    if (cs != cudaStreamCaptureStatusNone) {  // (an ILU(0) apply in a captured iteration: small blocks, which fit beside any)
+        YG_CUDA(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(threads), args, smem, ctx->stream));
+        YG_LAUNCHED(ctx);
+        return YG_OK;
+    }
     std::lock_guard<std::mutex> hold(m);
     if (last[d]) YG_CUDA(cudaStreamWaitEvent(ctx->stream, last[d], 0));
     else YG_CUDA(cudaEventCreateWithFlags(&last[d], cudaEventDisableTiming));
