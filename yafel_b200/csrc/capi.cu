@@ -530,6 +530,7 @@ extern "C" yg_status yg_matrix_destroy(yg_matrix A) {
     dev_free(ctx, A->d_corr32);
     dev_free(ctx, A->d_diag);
     for (int k = 0; k < 3; ++k) dev_free(ctx, A->d_ctiles[k]);
+    for (void *p : A->d_parts) dev_free(ctx, p);
     for (void *p : {(void *)A->d_bcmask, (void *)A->d_bcg, (void *)A->d_bcq, (void *)A->d_bcvals, (void *)A->d_bcdofs})
         dev_free(ctx, p);
     delete A;
@@ -606,18 +607,18 @@ extern "C" yg_status yg_spmv(yg_matrix A, yg_vector x, yg_vector y) { return yg_
 
 // Checks a (variant, lanes) choice for A and builds what it needs.
 static yg_status spmv_choice_check(yg_matrix A, int32_t variant, int32_t lanes) {
-    if (!A || variant < -1 || variant > 4 ||
+    if (!A || variant < -1 || variant > 5 ||
         (lanes != 1 && lanes != 2 && lanes != 4 && lanes != 8 && lanes != 16 && lanes != 32))
         return fail(YG_BAD_ARG, "yg_matrix_set_spmv: bad variant/lanes");
-    if ((variant == 1 || variant == 2 || variant == 4) && A->block != 2 && A->block != 3)
+    if ((variant == 1 || variant == 2 || variant >= 4) && A->block != 2 && A->block != 3)
         return fail(YG_UNSUPPORTED, "staged SpMV needs 2x2 or 3x3 blocks");
     if (variant == 0 && lanes == 1) return fail(YG_BAD_ARG, "flat SpMV needs 2..32 lanes");
-    if (variant == 3 || variant == 4) YG_TRY(spmv_prepare(A, variant, lanes));
+    if (variant >= 3) YG_TRY(spmv_prepare(A, variant, lanes));
     return YG_OK;
 }
 
 extern "C" yg_status yg_matrix_set_spmv_for(yg_matrix A, int32_t precision, int32_t variant, int32_t lanes) {
-    if (variant < 0) return fail(YG_BAD_ARG, "yg_matrix_set_spmv_for: a variant (0..4), not the autotuner");
+    if (variant < 0) return fail(YG_BAD_ARG, "yg_matrix_set_spmv_for: a variant (0..5), not the autotuner");
     YG_TRY(spmv_choice_check(A, variant, lanes));
     if (precision == YG_PREC_FP64) {
         A->variant = variant;

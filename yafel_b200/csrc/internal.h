@@ -112,7 +112,7 @@ struct yg_matrix_t {
     int32_t *d_diag = nullptr;    // position of the diagonal block in each block row, -1 if absent
     int lanes = 32;               // SpMV lanes per block row (flat variant)
     int variant = 0;              // SpMV variant: 0 flat lane-strided, 1 cp.async staged, 2 TMA bulk staged (B = 2, 3),
-                                  // 3 TMA row tiles (B = 1), 4 TMA whole rows (B = 2, 3)
+                                  // 3 TMA row tiles (B = 1), 4 TMA whole rows, 5 TMA block stream (B = 2, 3)
     int variant32 = -1, lanes32 = 32;  // choice for FP32 values (-1: as for FP64)
     bool tuned32 = false;
     bool tuned = false;
@@ -128,6 +128,8 @@ struct yg_matrix_t {
     // of each tile of at most (256 << k) entries, then the row count
     int32_t *d_ctiles[3] = {nullptr, nullptr, nullptr};
     int64_t nctiles[3] = {0, 0, 0};
+    // the warps' shares of the block-stream SpMV (variant 5): FP64 configurations, then FP32
+    void *d_parts[4] = {};
     int32_t row_min = -1, row_max = -1;  // entries per row, -1 until measured
     int64_t rows() const { return nbrows * block; }
     int64_t cols() const { return nbcols * block; }

@@ -17,6 +17,7 @@
 #include "internal.h"
 #include "device_common.cuh"
 
+#include <algorithm>
 #include <type_traits>
 #include <atomic>
 
@@ -844,6 +845,9 @@ static yg_status csr_tiles_build(yg_matrix A, int k) {
 
 static int rows_capacity_of(int lanes) { return lanes <= 2 ? 128 : 64; }
 
+static bool stream_lanes_ok(int lanes);
+static yg_status stream_parts_build(yg_matrix A, int lanes, bool f32);
+
 yg_status spmv_prepare(yg_matrix A, int variant, int lanes) {
     if (variant == 4) {  // whole rows: every block row must fit one stage
         if (lanes != 1 && lanes != 2 && lanes != 4 && lanes != 8)
@@ -855,6 +859,13 @@ yg_status spmv_prepare(yg_matrix A, int variant, int lanes) {
             return fail(YG_UNSUPPORTED, "whole-row SpMV (lanes %d) holds rows of up to %d blocks; the longest has %d",
                         lanes, rows_capacity_of(lanes), A->row_max);
         return YG_OK;
+    }
+    if (variant == 5) {  // block stream: the warps' shares, for both value types
+        if (!stream_lanes_ok(lanes)) return fail(YG_BAD_ARG, "block-stream SpMV configurations are lanes 1, 2");
+        if (A->block != 2 && A->block != 3) return fail(YG_UNSUPPORTED, "block-stream SpMV needs 2x2 or 3x3 blocks");
+        if (A->nbrows < 1 || A->nbrows >= INT32_MAX) return fail(YG_UNSUPPORTED, "block-stream SpMV needs 1 to 2^31 - 2 block rows");
+        YG_TRY(stream_parts_build(A, lanes, false));
+        return stream_parts_build(A, lanes, true);
     }
     if (variant != 3) return YG_OK;
     if (!csr_lanes_ok(lanes)) return fail(YG_BAD_ARG, "row-tile SpMV configurations are lanes 1, 2, 4, 8");
@@ -1233,6 +1244,405 @@ static void rows_shape_bv(int lanes, int *smem, int *wp) {
     }
 }
 
+// ---------------------------------------------------------------------------
+// Block-stream variant for B = 2, 3 (variant 5).  The variants above give a warp
+// whole rows.  That leaves lanes idle at every row's end (a row of 45 blocks takes
+// two steps of 32), costs a copy, a wait and a reduction per row, and balances
+// badly: a warp of a mid-size matrix gets five rows of 27 to 125 blocks, and the
+// slowest warp ends the kernel.  Here a warp streams an equal share of
+// consecutive blocks, whatever rows they belong to: stages of CH blocks by two
+// bulk copies, each lane one block of 32 at a time, its B products added to the
+// lane's sums of the current row; where a row ends inside the 32, the lanes below
+// the end add to it, the sums are reduced (the transposed butterfly) and written,
+// and the others begin the next row.  CTAs begin and end at rows; a row that
+// crosses warps of a CTA is put together at the end from the warps' partial sums,
+// in warp order.  The share of every warp and its first row are laid out once per
+// matrix (StreamPart, from the row pointers).  Sums have a fixed order.  Waits are
+// bounded as in the variants above.
+// Alone, best of the variants above -> this, 3x3 blocks: FP32 values with the
+// correction, 40^3 Q2 337 -> 281 us (4.7 TB/s), 30^3 146 -> 129, 14^3 Q3 (rows of up to
+// 343 blocks) 94 -> 73; FP64 40^3 419 -> 404 us (6.2 TB/s), 13^3 20.2 -> 18.6; 2x2
+// blocks, FP64 200^2 order 2 53 -> 44.  Rows of 27 blocks (48^3 Q1) stay with the chunked
+// kernel, 51 against 56: a step then ends a row or two, and reduces as often.
+struct alignas(16) StreamPart {
+    int32_t begin, end;  // the warp's blocks
+    int32_t row;         // its first row (bit 31: blocks of it come before `begin`)
+    int32_t row_end;     // one past the CTA's last row
+};
+
+template <int B, typename VT, int CH_, int NST_, int WARPS_, int CTAS_>
+struct StreamCfg {
+    static constexpr int CH = CH_, NST = NST_, WARPS = WARPS_, CTAS = CTAS_, U = CH / 32;
+    static constexpr int VBYTES = (CH * B * B * (int)sizeof(VT) + 32 + 15) & ~15;
+    static constexpr int CBYTES = (CH * 4 + 32 + 15) & ~15;
+    static constexpr int STAGE = VBYTES + CBYTES;
+    static constexpr int SMEM = WARPS * NST * STAGE + WARPS * NST * 8;  // stages + mbarriers
+};
+// Configurations, selected by the `lanes` field of a variant-5 matrix: 24 warps per
+// SM with the registers that leaves them beat 40 (48 registers, spilled), 32 and 16;
+// three stages of 32 blocks are best for FP64 values, two of 64 for FP32.
+template <int B, typename VT> using StreamL1 = StreamCfg<B, VT, 32, 3, 8, 3>;
+template <int B, typename VT> using StreamL2 = StreamCfg<B, VT, 64, 2, 4, 6>;
+static bool stream_lanes_ok(int lanes) { return lanes == 1 || lanes == 2; }
+
+template <int B, typename VT, int DOT, typename C, bool XF>
+__global__ void __launch_bounds__(C::WARPS * 32, C::CTAS)
+k_bcsr_spmv_stream(const StreamPart *__restrict__ parts, const int32_t *__restrict__ rowptr,
+                   const int32_t *__restrict__ col, const VT *__restrict__ val, const double *__restrict__ x,
+                   const float *__restrict__ x32, double *__restrict__ y, const double *__restrict__ w,
+                   double *__restrict__ partials, const int32_t *__restrict__ flag, const double *__restrict__ corr,
+                   int32_t *__restrict__ err) {
+    constexpr int B2 = B * B;
+    constexpr int BB = B2 * (int)sizeof(VT);
+    constexpr int GL = B == 2 ? 16 : 8;  // lanes per reduced component
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ double red[C::WARPS + 1];
+    __shared__ double head[C::WARPS][B], tail[C::WARPS][B];  // sums of a row begun before / not ended in the warp
+    __shared__ int head_row[C::WARPS], open_all[C::WARPS];   // its row (-1: none); no row ended in the warp
+    if (flag && read_flag(flag)) return;
+    const uint64_t pol = evict_first_policy();
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    unsigned char *ring = smem_raw + (size_t)wib * C::NST * C::STAGE;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem_raw + (size_t)C::WARPS * C::NST * C::STAGE) + wib * C::NST;
+    const int4 pt = __ldg(reinterpret_cast<const int4 *>(parts) + blockIdx.x * C::WARPS + wib);
+    const int begin = pt.x, end = pt.y, row_end = pt.w;
+    int row = pt.z & 0x7fffffff;
+    bool begun = pt.z < 0;  // the current row has blocks in the warps before
+    if (lane == 0) {
+        for (int k = 0; k < C::NST; ++k) mbar_init(&bars[k], 1);
+        head_row[wib] = -1;
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    __syncwarp();
+    const char *vbytes = reinterpret_cast<const char *>(val);
+    const char *cbytes = reinterpret_cast<const char *>(col);
+    auto issue = [&](int b, int st) {  // blocks [b, b + CH) of the share into stage st (an empty copy past the end)
+        if (lane == 0) {
+            const int n = min(C::CH, end - b);
+            if (n > 0) {
+                const int64_t vs = (int64_t)b * BB, va = vs & ~(int64_t)15, ve = (vs + (int64_t)n * BB + 15) & ~(int64_t)15;
+                const int64_t cs = (int64_t)b * 4, ca = cs & ~(int64_t)15, ce = (cs + (int64_t)n * 4 + 15) & ~(int64_t)15;
+                unsigned char *dst = ring + st * C::STAGE;
+                mbar_expect_tx(&bars[st], (unsigned)((ve - va) + (ce - ca)));
+                bulk_g2s(dst, vbytes + va, (unsigned)(ve - va), &bars[st], pol);
+                bulk_g2s(dst + C::VBYTES, cbytes + ca, (unsigned)(ce - ca), &bars[st], pol);
+            } else {
+                mbar_expect_tx(&bars[st], 0);  // completes the phase with no transfer
+            }
+        }
+    };
+#pragma unroll
+    for (int k = 0; k < C::NST - 1; ++k) issue(min(begin + k * C::CH, end), k);
+    // ends of the next 32 rows, lane k holding row base + k's
+    int base = row, ends = __ldg(rowptr + min(row + lane, row_end - 1) + 1);
+    int rend = __shfl_sync(0xffffffffu, ends, 0);
+    const int comp = lane / GL;  // the sum this lane holds after a reduction
+    const bool writer = (lane % GL) == 0 && comp < B;
+    double cr[B], xr[B];  // the current row's correction and own x, fetched when it begins
+    auto fetch = [&]() {
+        if (corr && writer && row < row_end) {
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                cr[k] = corr[((int64_t)row * B + comp) * B + k];
+                xr[k] = x[(int64_t)row * B + k];
+            }
+        }
+    };
+    fetch();
+    double acc[B], dot = 0, yy = 0;
+#pragma unroll
+    for (int i = 0; i < B; ++i) acc[i] = 0;
+    auto put = [&](double s, int64_t r, int i) {  // component i of row r
+        const int64_t yi = r * B + i;
+        y[yi] = s;
+        if (DOT >= 1) dot = fma(s, w[yi], dot);
+        if (DOT == 2) yy = fma(s, s, yy);
+    };
+    bool ended = false;  // a row ended in this warp
+    auto end_row = [&]() {
+        double s = reduce_rows_t<B>(acc, lane);
+        if (writer) {
+            if (begun) {
+                head[wib][comp] = s;
+                if (comp == 0) head_row[wib] = row;
+            } else {
+                if (corr) {
+                    double t = cr[0] * xr[0];
+#pragma unroll
+                    for (int k = 1; k < B; ++k) t = fma(cr[k], xr[k], t);
+                    s += t;
+                }
+                put(s, row, comp);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < B; ++i) acc[i] = 0;
+        begun = false;
+        ended = true;
+        ++row;
+        if (row - base == 32) {
+            base = row;
+            ends = __ldg(rowptr + min(row + lane, row_end - 1) + 1);
+        }
+        rend = __shfl_sync(0xffffffffu, ends, row - base);
+        fetch();
+    };
+    int st = 0;
+    unsigned phase = 0;  // bit k: parity of stage k's next completion
+    bool timed_out = false;
+    for (int b = begin; b < end; b += C::CH) {
+        issue(min(b + (C::NST - 1) * C::CH, end), (st + C::NST - 1) % C::NST);
+        int ok = 1;
+        if (lane == 0) {
+            long long spins = 0;
+            while (!mbar_try_wait(&bars[st], (phase >> st) & 1u))
+                if (++spins > kSpinLimit) { ok = 0; break; }
+        }
+        ok = __shfl_sync(0xffffffffu, ok, 0);
+        if (!ok) { timed_out = true; break; }
+        if (lane != 0) mbar_try_wait(&bars[st], (phase >> st) & 1u);
+        phase ^= (1u << st);
+        __syncwarp();
+        const unsigned char *stg = ring + st * C::STAGE;
+        const VT *blk = reinterpret_cast<const VT *>(stg + (((unsigned)b * (unsigned)BB) & 15u));
+        const int32_t *cix = reinterpret_cast<const int32_t *>(stg + C::VBYTES + (((unsigned)b * 4u) & 15u));
+        const int n = min(C::CH, end - b);
+        double t[C::U][B];
+        {
+            double xv[C::U][B];
+#pragma unroll
+            for (int u = 0; u < C::U; ++u) {
+                const int j = min(lane + 32 * u, n - 1);
+                gather_x<B, XF>(x, x32, cix[j], xv[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < C::U; ++u) {
+                const int j = min(lane + 32 * u, n - 1);
+#pragma unroll
+                for (int i = 0; i < B; ++i) {
+                    t[u][i] = (double)blk[j * B2 + i * B] * xv[u][0];
+#pragma unroll
+                    for (int k = 1; k < B; ++k) t[u][i] = fma((double)blk[j * B2 + i * B + k], xv[u][k], t[u][i]);
+                }
+            }
+        }
+        __syncwarp();  // the stage is free again
+        int pos = 0;   // blocks of the stage already added
+        while (row < row_end && rend - b <= n) {  // a row ends in the stage
+            const int e = rend - b;
+#pragma unroll
+            for (int u = 0; u < C::U; ++u) {
+                const int j = lane + 32 * u;
+                if (j >= pos && j < e) {
+#pragma unroll
+                    for (int i = 0; i < B; ++i) acc[i] += t[u][i];
+                }
+            }
+            pos = e;
+            end_row();
+        }
+#pragma unroll
+        for (int u = 0; u < C::U; ++u) {
+            const int j = lane + 32 * u;
+            if (j >= pos && j < n) {
+#pragma unroll
+                for (int i = 0; i < B; ++i) acc[i] += t[u][i];
+            }
+        }
+        st = (st + 1) % C::NST;
+    }
+    if (!timed_out)
+        while (row < row_end && rend <= end) end_row();  // rows without blocks behind the last one
+    {
+        const double s = reduce_rows_t<B>(acc, lane);
+        if (writer) tail[wib][comp] = s;
+        if (lane == 0) open_all[wib] = !ended;
+    }
+    if (timed_out && lane == 0 && err) atomicExch(err, (int32_t)YG_TIMEOUT);
+    // drain the copies still in flight into this warp's stages (bounded): NST-1
+    // after the loop, all NST after a timeout (the failed stage included)
+    if (lane == 0) {
+        const int outstanding = timed_out ? C::NST : C::NST - 1;
+        for (int k = 0; k < outstanding; ++k) {
+            const int s2 = (st + k) % C::NST;
+            long long spins = 0;
+            while (!mbar_try_wait(&bars[s2], (phase >> s2) & 1u) && ++spins <= kSpinLimit) {
+            }
+            phase ^= (1u << s2);
+        }
+    }
+    __syncthreads();
+    // rows that cross warps, by the warp in which they end: the sums of the warps
+    // before, in order, then its own
+    if (wib == 0 && lane < C::WARPS && head_row[lane] >= 0) {
+        int first = lane - 1;
+        while (first > 0 && open_all[first]) --first;
+        const int64_t r = head_row[lane];
+#pragma unroll
+        for (int i = 0; i < B; ++i) {
+            double s = 0;
+            for (int k = first; k < lane; ++k) s += tail[k][i];
+            s += head[lane][i];
+            if (corr) {
+                double c = corr[(r * B + i) * B] * x[r * B];
+#pragma unroll
+                for (int k = 1; k < B; ++k) c = fma(corr[(r * B + i) * B + k], x[r * B + k], c);
+                s += c;
+            }
+            put(s, r, i);
+        }
+    }
+    __syncwarp();
+    if (DOT) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            dot += __shfl_xor_sync(0xffffffffu, dot, o);
+            if (DOT == 2) yy += __shfl_xor_sync(0xffffffffu, yy, o);
+        }
+        if (lane == 0) red[wib] = dot;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double sum = 0;
+            for (int i = 0; i < C::WARPS; ++i) sum += red[i];
+            if (DOT == 1) partials[blockIdx.x] = sum;
+            else partials[2 * blockIdx.x] = sum;
+        }
+        if (DOT == 2) {
+            __syncthreads();
+            if (lane == 0) red[wib] = yy;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                double sum = 0;
+                for (int i = 0; i < C::WARPS; ++i) sum += red[i];
+                partials[2 * blockIdx.x + 1] = sum;
+            }
+        }
+    }
+}
+
+// Shares of the block-stream variant: CTA c takes the rows whose first block lies in
+// [c nnzb / G, (c + 1) nnzb / G) (the first CTA also those before, the last those
+// behind), its warps equal runs of their blocks in whole steps of 32.
+__global__ void k_stream_parts(int64_t nbrows, int64_t nnzb, int G, int warps, const int32_t *__restrict__ rowptr,
+                               StreamPart *__restrict__ parts) {
+    auto first_at = [&](int64_t target) {  // first row with rowptr[row] >= target
+        int64_t lo = 0, hi = nbrows;
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (rowptr[mid] < target) lo = mid + 1;
+            else hi = mid;
+        }
+        return lo;
+    };
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < G * warps; i += gridDim.x * blockDim.x) {
+        const int c = i / warps, w = i - c * warps;
+        const int64_t r0 = c == 0 ? 0 : first_at(c * nnzb / G), r1 = c + 1 == G ? nbrows : first_at((c + 1) * nnzb / G);
+        const int64_t b0 = rowptr[r0], b1 = rowptr[r1];
+        const int64_t per = ((b1 - b0 + warps - 1) / warps + 31) / 32 * 32;
+        StreamPart p;
+        p.begin = (int32_t)min(b0 + w * per, b1);
+        p.end = (int32_t)min(b0 + (w + 1) * per, b1);
+        p.row_end = (int32_t)r1;
+        int64_t row = r0;
+        if (w > 0) {  // first row that ends behind `begin` (rows that end there belong to the warps before)
+            int64_t lo = r0, hi = r1;
+            while (lo < hi) {
+                const int64_t mid = (lo + hi) >> 1;
+                if (rowptr[mid + 1] <= p.begin) lo = mid + 1;
+                else hi = mid;
+            }
+            row = lo;
+        }
+        p.row = (int32_t)row | (row < r1 && rowptr[row] < p.begin ? (int32_t)0x80000000 : 0);
+        parts[i] = p;
+    }
+}
+
+template <int B, typename VT>
+static void stream_shape_bv(int lanes, int *smem, int *wp, int *ctas) {
+    switch (lanes) {
+    case 1: shape_of<StreamL1<B, VT>>(smem, wp); *ctas = StreamL1<B, VT>::CTAS; break;
+    default: shape_of<StreamL2<B, VT>>(smem, wp); *ctas = StreamL2<B, VT>::CTAS; break;
+    }
+}
+
+// Grid and warps per CTA of a configuration: one wave, as many CTAs per SM as the
+// shared memory holds (within the registers of its launch bounds), no more warps than steps.
+static void stream_grid_of(yg_matrix A, int lanes, bool f32, int *grid, int *warps) {
+    int smem = 0, ctas = 1;
+    if (A->block == 3) {
+        if (f32) stream_shape_bv<3, float>(lanes, &smem, warps, &ctas);
+        else stream_shape_bv<3, double>(lanes, &smem, warps, &ctas);
+    } else {
+        if (f32) stream_shape_bv<2, float>(lanes, &smem, warps, &ctas);
+        else stream_shape_bv<2, double>(lanes, &smem, warps, &ctas);
+    }
+    const int per = std::max(1, std::min(ctas, (220 * 1024) / (smem + 1024)));
+    const int64_t steps = (A->nnzb + 31) / 32;
+    *grid = (int)std::max<int64_t>(1, std::min<int64_t>((steps + *warps - 1) / *warps, (int64_t)A->ctx->num_sms * per));
+}
+
+// The shares of configuration `lanes` for one value type, laid out on first use.
+static yg_status stream_parts_build(yg_matrix A, int lanes, bool f32) {
+    yg_context ctx = A->ctx;
+    const int slot = 2 * (f32 ? 1 : 0) + lanes - 1;
+    if (A->d_parts[slot]) return YG_OK;
+    cudaStreamCaptureStatus cs;
+    YG_CUDA(cudaStreamIsCapturing(ctx->stream, &cs));
+    if (cs != cudaStreamCaptureStatusNone) return fail(YG_BAD_ARG, "SpMV shares cannot be laid out during stream capture");
+    int grid, warps;
+    stream_grid_of(A, lanes, f32, &grid, &warps);
+    StreamPart *p = nullptr;
+    YG_TRY(dev_alloc_t(ctx, &p, (size_t)grid * warps));
+    k_stream_parts<<<(grid * warps + kThreads - 1) / kThreads, kThreads, 0, ctx->stream>>>(A->nbrows, A->nnzb, grid, warps,
+                                                                                          A->d_rowptr, p);
+    YG_LAUNCHED(ctx);
+    YG_CUDA(cudaGetLastError());
+    A->d_parts[slot] = p;
+    return YG_OK;
+}
+
+template <int B, typename VT, int DOT, typename C, bool XF>
+static yg_status launch_stream_xf(yg_matrix A, int lanes, const VT *val, const double *x, const float *x32, double *y,
+                                  const double *w, double *partials, const int32_t *flag, const double *corr,
+                                  cudaStream_t st) {
+    static std::atomic<uint64_t> attr{0};
+    if (smem_attr_due(attr, A->ctx->device)) {
+        cudaFuncSetAttribute(k_bcsr_spmv_stream<B, VT, DOT, C, XF>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+        smem_attr_done(attr, A->ctx->device);
+    }
+    constexpr bool f32 = std::is_same<VT, float>::value;
+    const int slot = 2 * (f32 ? 1 : 0) + lanes - 1;
+    if (!A->d_parts[slot]) return fail(YG_BAD_ARG, "block-stream SpMV launched without its shares (lanes %d)", lanes);
+    int grid, warps;  // the shares' grid, whatever the caller's
+    stream_grid_of(A, lanes, f32, &grid, &warps);
+    k_bcsr_spmv_stream<B, VT, DOT, C, XF><<<grid, C::WARPS * 32, C::SMEM, st>>>(
+        static_cast<const StreamPart *>(A->d_parts[slot]), A->d_rowptr, A->d_col, val, x, x32, y, w, partials, flag, corr,
+        A->ctx->d_err);
+    YG_LAUNCHED(A->ctx);
+    return YG_OK;
+}
+
+template <int B, typename VT, int DOT, typename C>
+static yg_status launch_stream_cfg(yg_matrix A, int lanes, const VT *val, const double *x, const float *x32, double *y,
+                                   const double *w, double *partials, const int32_t *flag, const double *corr,
+                                   cudaStream_t st) {
+    if constexpr (std::is_same<VT, float>::value) {
+        if (x32) return launch_stream_xf<B, VT, DOT, C, true>(A, lanes, val, x, x32, y, w, partials, flag, corr, st);
+    }
+    return launch_stream_xf<B, VT, DOT, C, false>(A, lanes, val, x, nullptr, y, w, partials, flag, corr, st);
+}
+
+template <int B, typename VT, int DOT>
+static yg_status launch_stream(yg_matrix A, int lanes, const VT *val, const double *x, const float *x32, double *y,
+                               const double *w, double *partials, const int32_t *flag, const double *corr,
+                               cudaStream_t st) {
+    switch (lanes) {
+    case 1: return launch_stream_cfg<B, VT, DOT, StreamL1<B, VT>>(A, lanes, val, x, x32, y, w, partials, flag, corr, st);
+    default: return launch_stream_cfg<B, VT, DOT, StreamL2<B, VT>>(A, lanes, val, x, x32, y, w, partials, flag, corr, st);
+    }
+}
+
 // CTAs per SM and warps per CTA of a TMA configuration (for the grid size): as
 // many CTAs as the shared memory holds, at most 64 warps and 8 CTAs per SM (the
 // Krylov kernels reserve 8 partial sums per SM for the SpMV).
@@ -1286,6 +1696,10 @@ static yg_status launch_b(yg_matrix A, int variant, int lanes, const VT *val, co
                           double *y, const double *w, double *partials, const int32_t *flag, const double *corr, int grid,
                           cudaStream_t st) {
     if (variant == 3) return launch_csr<VT, DOT>(A, lanes, val, x, y, w, partials, flag, corr, grid, st);
+    if (variant == 5 && A->block == 3)
+        return launch_stream<3, VT, DOT>(A, lanes, val, x, x32, y, w, partials, flag, corr, st);
+    if (variant == 5 && A->block == 2)
+        return launch_stream<2, VT, DOT>(A, lanes, val, x, x32, y, w, partials, flag, corr, st);
     if (variant == 4 && A->block == 3)
         return launch_rows<3, VT, DOT>(A, lanes, val, x, x32, y, w, partials, flag, corr, grid, st);
     if (variant == 4 && A->block == 2)
@@ -1401,6 +1815,11 @@ int spmv_grid_for(yg_matrix A, int precision) {
         if (need < g) g = need;
         return (int)(g < 1 ? 1 : g);
     }
+    if (variant == 5) {  // block stream: the grid its shares were laid out for
+        int grid, warps;
+        stream_grid_of(A, lanes, f32, &grid, &warps);
+        return grid;
+    }
     if (variant == 4) {  // whole rows: as many CTAs as the shared memory holds, a warp per row
         int smem = 0, wp = 1;
         if (A->block == 3) {
@@ -1484,6 +1903,8 @@ static yg_status tune_precision(yg_matrix A, int precision, double *x, const flo
         for (int L : {32, 1, 2, 4, 8, 16}) cands.push_back({2, L});  // TMA configurations
         for (int L : {1, 2, 4, 8})  // whole-row configurations, where the longest row fits a stage
             if (spmv_prepare(A, 4, L) == YG_OK) cands.push_back({4, L});
+        for (int L : {1, 2})  // block-stream configurations
+            if (spmv_prepare(A, 5, L) == YG_OK) cands.push_back({5, L});
     }
     const bool f32 = precision != YG_PREC_FP64;
     const double *corr = f32 ? A->d_corr32 : nullptr;
