@@ -41,6 +41,28 @@ __device__ __forceinline__ double reduce_partials(const double *__restrict__ par
     return block_sum_all<NT>(s, sm);
 }
 
+// Sums of NT threads' values of v0 and v1 (the order of block_sum), in every thread;
+// sm: 2 * NT / 32 doubles that no thread touches before the next barrier.
+template <int NT>
+__device__ __forceinline__ void block_sum2_all(double &v0, double &v1, double *sm) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+        v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        sm[threadIdx.x >> 5] = v0;
+        sm[NT / 32 + (threadIdx.x >> 5)] = v1;
+    }
+    __syncthreads();
+    v0 = v1 = 0;
+#pragma unroll
+    for (int i = 0; i < NT / 32; ++i) {
+        v0 += sm[i];
+        v1 += sm[NT / 32 + i];
+    }
+}
+
 // Streaming loads for matrix values: read once per SpMV, so they bypass L1 and
 // carry an L2 evict-first policy, which keeps the gathered vector resident.
 __device__ __forceinline__ uint64_t evict_first_policy() {

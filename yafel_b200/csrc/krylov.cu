@@ -3,18 +3,19 @@
 // Replaces cg_solve (solver/iterative/cg_solve.hpp:23-81), pcg_solve
 // (pcg_solve.hpp:115-178) and bicgstab_solve (bicgstab_solve.hpp:207-283).
 //
-// One PCG iteration is three kernels on a persistent grid of G blocks:
+// One PCG iteration is three kernels:
 //   1. q = A p fused with per-block partials of p.q                (spmv.cu)
-//   2. every block reduces the G partials in the same order -> alpha;
+//   2. every block reduces those partials in the same order -> alpha;
 //      x += alpha p, r -= alpha q, z = M^-1 r (Jacobi fused), partials of r.z, r.r
 //   3. every block reduces those -> beta; p = z + beta p; block 0 records the
 //      scalars and the convergence flag.
 // Scalars live in device memory (KrylovScalars); r.z is double-buffered by
 // iteration parity so no block reads a value another block of the same kernel
-// is writing.  A run of iterations is captured once into a CUDA graph and
-// replayed; kernels return immediately once the flag is set, and the host reads
-// the flag once per replay.  Systems whose matrix fits the shared memory of the SMs
-// run the same iteration in one cooperative kernel instead (pcg_resident.cu).  All reductions have a fixed order, so a solve is
+// is writing.  Kernels return immediately once the flag is set, and the host reads
+// the flag once per check_every iterations.  The first two such runs are launched
+// kernel by kernel, the later ones replay a captured graph.  Systems whose matrix
+// fits the shared memory of the SMs run the same iteration in one cooperative kernel
+// instead (pcg_resident.cu).  All reductions have a fixed order, so a solve is
 // bit-reproducible.  ILU(0) goes through the general path (z stored, apply by
 // precond.cu, then a separate r.z reduction).
 #include "internal.h"
@@ -119,13 +120,34 @@ k_cg_scalars_replace(KrylovScalars *S, const double *__restrict__ partials, int 
 
 // Kernel 2 of the iteration.  JAC: z = dinv*r computed in registers (M is
 // Jacobi or identity); otherwise only r.r partials (z comes from M later).
+// Small systems are bound by the latency of two dependent passes, partials then
+// vectors, so the vectors' first loads are issued before the partials are added and
+// the two sums of a block share one barrier; large ones are bound by HBM either way.
+// With this, the same in k_cg_pupdate and the grid below, one FP64 iteration went from
+// 20.1 to 17.2 us at 27,783 rows, 37.0 to 34.8 at 89,373, 32.3 to 30.4 at 361,201
+// (9 entries a row) and 191 to 190 at 680,943.
 template <bool FUSED>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 4)
 k_cg_update(int64_t n, const double *__restrict__ pq_partials, int np, KrylovScalars *S, int parity,
             double *__restrict__ x, double *__restrict__ r, const double *__restrict__ p,
             const double *__restrict__ q, const double *__restrict__ dinv, double *__restrict__ partials_out) {
-    __shared__ double sm[kThreads / 32 + 1];
+    __shared__ double sm[kThreads / 32 + 1], sm2[2 * (kThreads / 32)];
     if (read_flag(&S->flag)) return;
+    int64_t lo, hi;
+    block_chunk2(n, lo, hi);
+    const int64_t v1 = hi >> 1;
+    // pairs of entries as 16-byte loads (the chunk starts on an even index); the
+    // first pair is on its way while the partials are added
+    int64_t v = (lo >> 1) + threadIdx.x;
+    double2 xv, pv, rv, qv, dv;
+    auto load = [&](int64_t i) {
+        xv = reinterpret_cast<const double2 *>(x)[i];
+        pv = reinterpret_cast<const double2 *>(p)[i];
+        rv = reinterpret_cast<const double2 *>(r)[i];
+        qv = reinterpret_cast<const double2 *>(q)[i];
+        if (FUSED && dinv) dv = reinterpret_cast<const double2 *>(dinv)[i];
+    };
+    if (v < v1) load(v);
     const double pq = reduce_partials<kThreads>(pq_partials, np, 1, 0, sm);
     const double alpha = S->rz[parity] / pq;
     // no definiteness test: the reference runs CG on negative definite systems
@@ -135,10 +157,7 @@ k_cg_update(int64_t n, const double *__restrict__ pq_partials, int np, KrylovSca
         return;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) S->iter_seen = S->iter;  // for k_cg_pupdate's iteration cap test
-    int64_t lo, hi;
-    block_chunk2(n, lo, hi);
     double srz = 0, srr = 0;
-    // pairs of entries as 16-byte loads (the chunk starts on an even index)
     auto one = [&](int64_t i) {
         x[i] += p[i] * alpha;
         double ri = r[i] + (-alpha) * q[i];
@@ -149,13 +168,7 @@ k_cg_update(int64_t n, const double *__restrict__ pq_partials, int np, KrylovSca
             srz += ri * zi;
         }
     };
-    const int64_t v1 = hi >> 1;
-#pragma unroll 2
-    for (int64_t v = (lo >> 1) + threadIdx.x; v < v1; v += blockDim.x) {
-        double2 xv = reinterpret_cast<const double2 *>(x)[v];
-        const double2 pv = reinterpret_cast<const double2 *>(p)[v];
-        double2 rv = reinterpret_cast<const double2 *>(r)[v];
-        const double2 qv = reinterpret_cast<const double2 *>(q)[v];
+    while (v < v1) {
         xv.x += pv.x * alpha;
         xv.y += pv.y * alpha;
         rv.x = rv.x + (-alpha) * qv.x;
@@ -167,17 +180,17 @@ k_cg_update(int64_t n, const double *__restrict__ pq_partials, int np, KrylovSca
         if (FUSED) {
             double2 zv = rv;
             if (dinv) {
-                const double2 dv = reinterpret_cast<const double2 *>(dinv)[v];
                 zv.x = dv.x * rv.x;
                 zv.y = dv.y * rv.y;
             }
             srz += rv.x * zv.x;
             srz += rv.y * zv.y;
         }
+        v += blockDim.x;
+        if (v < v1) load(v);
     }
     if ((hi & 1) && hi > lo && threadIdx.x == 0) one(hi - 1);  // odd n: the last entry
-    srr = block_sum<kThreads>(srr, sm);
-    if (FUSED) srz = block_sum<kThreads>(srz, sm);
+    block_sum2_all<kThreads>(srz, srr, sm2);
     if (threadIdx.x == 0) {
         partials_out[2 * blockIdx.x + 0] = srz;
         partials_out[2 * blockIdx.x + 1] = srr;
@@ -198,14 +211,30 @@ struct Dir32 {
 };
 
 template <bool FUSED>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 4)
 k_cg_pupdate(int64_t n, const double *__restrict__ partials_in, int np, KrylovScalars *S, int parity,
              double *__restrict__ p, const double *__restrict__ r, const double *__restrict__ z,
              const double *__restrict__ dinv, Dir32 d32) {
-    __shared__ double sm[kThreads / 32 + 1];
+    __shared__ double sm[2 * (kThreads / 32)];
     if (read_flag(&S->flag)) return;
-    const double rz_new = reduce_partials<kThreads>(partials_in, np, 2, 0, sm);
-    const double rr = reduce_partials<kThreads>(partials_in, np, 2, 1, sm);
+    int64_t lo, hi;
+    block_chunk2(n, lo, hi);
+    const int64_t v1 = hi >> 1;
+    int64_t v = (lo >> 1) + threadIdx.x;  // the first pair is on its way while the partials are added
+    double2 rv, dv, pv;
+    auto load = [&](int64_t i) {
+        rv = reinterpret_cast<const double2 *>(FUSED ? r : z)[i];
+        if (FUSED && dinv) dv = reinterpret_cast<const double2 *>(dinv)[i];
+        pv = reinterpret_cast<const double2 *>(p)[i];
+    };
+    if (v < v1) load(v);
+    double rz_new = 0, rr = 0;
+    for (int i = threadIdx.x; i < np; i += kThreads) {
+        const double2 t = reinterpret_cast<const double2 *>(partials_in)[i];
+        rz_new += t.x;
+        rr += t.y;
+    }
+    block_sum2_all<kThreads>(rz_new, rr, sm);
     const double rz_old = S->rz[parity];
     // convergence test before the direction update, as the reference does
     bool done = false;
@@ -228,24 +257,19 @@ k_cg_pupdate(int64_t n, const double *__restrict__ partials_in, int np, KrylovSc
     }
     if (done) return;
     const double beta = rz_new / rz_old;
-    int64_t lo, hi;
-    block_chunk2(n, lo, hi);
-    const int64_t v1 = hi >> 1;
-#pragma unroll 2
-    for (int64_t v = (lo >> 1) + threadIdx.x; v < v1; v += blockDim.x) {
-        const double2 rv = reinterpret_cast<const double2 *>(FUSED ? r : z)[v];
+    while (v < v1) {
         double2 zv = rv;
         if (FUSED && dinv) {
-            const double2 dv = reinterpret_cast<const double2 *>(dinv)[v];
             zv.x = dv.x * rv.x;
             zv.y = dv.y * rv.y;
         }
-        double2 pv = reinterpret_cast<const double2 *>(p)[v];
         pv.x = zv.x + beta * pv.x;
         pv.y = zv.y + beta * pv.y;
         reinterpret_cast<double2 *>(p)[v] = pv;
         d32.put(2 * v, pv.x);
         d32.put(2 * v + 1, pv.y);
+        v += blockDim.x;
+        if (v < v1) load(v);
     }
     if ((hi & 1) && hi > lo && threadIdx.x == 0) {  // odd n: the last entry
         const int64_t i = hi - 1;
@@ -406,8 +430,12 @@ static yg_status pcg_core(yg_matrix A, yg_precond M, const double *b, double *x,
     const bool fused = !M || precond_fusable(M);
     const double *dinv = M ? precond_dinv(M) : nullptr;
     const int G = ctx->reduce_blocks;
+    // the update kernels' blocks: one pass of pairs each, at least one per SM: every
+    // block adds all blocks' partials (89,373 rows: 34.7 us an iteration with 175
+    // blocks, 36.4 with 592; 1,594,323 rows: 485 with 592, 492 with 148)
+    const int GU = (int)std::max<int64_t>(std::min<int64_t>(ctx->num_sms, G), std::min<int64_t>(G, (n + 2 * kThreads - 1) / (2 * kThreads)));
     const int spmv_grid = std::min(spmv_grid_for(A, precision), kMaxReduceBlocks);
-    double *P = ctx->d_partials;  // [0,G): p.q ; [2G,4G): r.z/r.r pairs ; [4G, 7G): init triples
+    double *P = ctx->d_partials;  // [0,2G): p.q ; [2G,4G): r.z/r.r pairs ; [4G, 7G): init triples
     KrylovScalars *S = ctx->d_scalars;
     cudaStream_t st = ctx->stream;
     // the FP32 direction copy serves the FP32-value iteration SpMV only; so does
@@ -443,17 +471,17 @@ static yg_status pcg_core(yg_matrix A, yg_precond M, const double *b, double *x,
         if (prof && prof->on) YG_CUDA(cudaEventRecordWithFlags(prof->stop[slot], st, cudaEventRecordExternal));
         ++slot;
         if (fused) {
-            k_cg_update<true><<<G, kThreads, 0, st>>>(n, P, spmv_grid, S, parity, x, w.r, w.p, w.q, dinv, P + 2 * G);
+            k_cg_update<true><<<GU, kThreads, 0, st>>>(n, P, spmv_grid, S, parity, x, w.r, w.p, w.q, dinv, P + 2 * G);
             YG_LAUNCHED(ctx);
-            k_cg_pupdate<true><<<G, kThreads, 0, st>>>(n, P + 2 * G, G, S, parity, w.p, w.r, nullptr, dinv, d32);
+            k_cg_pupdate<true><<<GU, kThreads, 0, st>>>(n, P + 2 * G, GU, S, parity, w.p, w.r, nullptr, dinv, d32);
             YG_LAUNCHED(ctx);
         } else {
-            k_cg_update<false><<<G, kThreads, 0, st>>>(n, P, spmv_grid, S, parity, x, w.r, w.p, w.q, nullptr, P + 2 * G);
+            k_cg_update<false><<<GU, kThreads, 0, st>>>(n, P, spmv_grid, S, parity, x, w.r, w.p, w.q, nullptr, P + 2 * G);
             YG_LAUNCHED(ctx);
             YG_TRY(precond_apply_dev(M, w.r, w.z, &S->flag));
-            k_dot2_partials<<<G, kThreads, 0, st>>>(n, w.r, w.z, P + 2 * G, &S->flag, 0, 2);
+            k_dot2_partials<<<GU, kThreads, 0, st>>>(n, w.r, w.z, P + 2 * G, &S->flag, 0, 2);
             YG_LAUNCHED(ctx);
-            k_cg_pupdate<false><<<G, kThreads, 0, st>>>(n, P + 2 * G, G, S, parity, w.p, w.r, w.z, nullptr, d32);
+            k_cg_pupdate<false><<<GU, kThreads, 0, st>>>(n, P + 2 * G, GU, S, parity, w.p, w.r, w.z, nullptr, d32);
             YG_LAUNCHED(ctx);
         }
         return YG_OK;
@@ -485,7 +513,11 @@ static yg_status pcg_core(yg_matrix A, yg_precond M, const double *b, double *x,
     if (hs.flag == FLAG_RUN || (hs.flag == FLAG_CONVERGED && criterion == YG_CRIT_RELRES && hs.iter > 0)) {
         IterGraph g;
         if (prof && prof->on && prof->start.empty()) YG_TRY(prof->init(check_every));
-        if (!w.zp) YG_TRY(capture(ctx, check_every, one, g));
+        // The first iterations go straight to the stream: a short solve captures no graph,
+        // which takes longer than the launches it saves (2 iterations took 0.55 ms with a
+        // graph and 0.19 without at 27,783 rows, 24 took 0.96 and 0.68 ms; at 1,594,323
+        // rows 12.2 and 11.9).  The event pairs of a profile belong to the graph.
+        const int64_t direct_its = prof && prof->on ? 0 : 2 * check_every;
         double rr_last = hs.rr;  // r.r at the last replacement
         int false_stops = 0;
         for (;;) {
@@ -493,7 +525,11 @@ static yg_status pcg_core(yg_matrix A, yg_precond M, const double *b, double *x,
             if (w.zp) {
                 YG_TRY(pcg_resident_launch(A, f32, dinv, x, w.r, w.p, w.zp, 1 << 12, check_every,
                                            reliable ? 1e-2 * rr_last : 0.0));
+            } else if (before < direct_its) {
+                for (int it = 0; it < check_every && before + it < maxiter; ++it) YG_TRY(one(it & 1));
+                YG_CUDA(cudaGetLastError());
             } else {
+                if (!g.exec) YG_TRY(capture(ctx, check_every, one, g));
                 YG_CUDA(cudaGraphLaunch(g.exec, st));
                 ctx->launches += g.kernels;
             }
