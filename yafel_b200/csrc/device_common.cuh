@@ -63,6 +63,19 @@ __device__ __forceinline__ void block_sum2_all(double &v0, double &v1, double *s
     }
 }
 
+// Every block sums the np pairs of partials in the same order; sm as in block_sum2_all.
+template <int NT>
+__device__ __forceinline__ void reduce_partials2(const double *__restrict__ partials, int np, double &a, double &b,
+                                                 double *sm) {
+    a = b = 0;
+    for (int i = threadIdx.x; i < np; i += NT) {
+        const double2 t = reinterpret_cast<const double2 *>(partials)[i];
+        a += t.x;
+        b += t.y;
+    }
+    block_sum2_all<NT>(a, b, sm);
+}
+
 // Streaming loads for matrix values: read once per SpMV, so they bypass L1 and
 // carry an L2 evict-first policy, which keeps the gathered vector resident.
 __device__ __forceinline__ uint64_t evict_first_policy() {

@@ -228,13 +228,8 @@ k_cg_pupdate(int64_t n, const double *__restrict__ partials_in, int np, KrylovSc
         pv = reinterpret_cast<const double2 *>(p)[i];
     };
     if (v < v1) load(v);
-    double rz_new = 0, rr = 0;
-    for (int i = threadIdx.x; i < np; i += kThreads) {
-        const double2 t = reinterpret_cast<const double2 *>(partials_in)[i];
-        rz_new += t.x;
-        rr += t.y;
-    }
-    block_sum2_all<kThreads>(rz_new, rr, sm);
+    double rz_new, rr;
+    reduce_partials2<kThreads>(partials_in, np, rz_new, rr, sm);
     const double rz_old = S->rz[parity];
     // convergence test before the direction update, as the reference does
     bool done = false;
