@@ -112,6 +112,8 @@ def test_sizes_about_the_shared_memory_of_the_gpu(ctx, n):
         x, st = yb.solve(K, F, M=M, tol=1e-10, precision=prec)
         xp, sp = yb.solve(K, F, M=M, tol=1e-10, precision=prec, profile=True)
         assert st.status == 0 and sp.status == 0
-        assert abs(sp.iterations - st.iterations) <= 2 + st.iterations // 20
+        # (FP32 values: counts follow the order of the sums, and a residual is replaced at
+        # every 16th iteration only: the streaming kernels themselves take 320 to 335)
+        assert abs(sp.iterations - st.iterations) <= (2 if prec == yb.PREC_FP64 else 16) + st.iterations // 20
         r = F.numpy() - (K * x.numpy())
         assert np.linalg.norm(r) <= 1.01e-10 * np.linalg.norm(F.numpy())

@@ -20,7 +20,9 @@
 //   S2  BiCGSTAB SpMV t = A sh (partials of t.s, t.t -> omega)
 //   V3  PCG: p = z + beta p; BiCGSTAB: x += alpha ph + omega sh, r = s - omega t,
 //       partials of r0.r, r.r -> beta and the stopping tests
-// (V1 and S2 are launched only when BiCGSTAB systems are present).  Every
+// (V1 and S2 are launched only when BiCGSTAB systems are present).  PCG systems that
+// fit the shared memory of the SMs run their iterations in one cooperative kernel
+// instead (k_batch_resident).  Every
 // decision about a system is taken once, by the warp or CTA that completes the
 // system's last item of a kernel (a per-system ticket; systems with more than
 // kChunk matrix items sum their partials in two levels), so every CTA of the
@@ -41,6 +43,7 @@
 // does not change.
 #include "internal.h"
 #include "device_common.cuh"
+#include "resident.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -49,6 +52,7 @@
 
 namespace yg {
 int stream_grid(yg_context ctx, int64_t n);
+yg_status launch_cooperative(yg_context ctx, const void *kern, int grid, int threads, size_t smem, void **args);
 }
 
 enum BatchFlag : int32_t { BF_RUN = 0, BF_DONE = 1, BF_BREAK = 2, BF_NANF = 3, BF_MAXIT = 4, BF_INIT = 5, BF_EMPTY = 6 };
@@ -72,6 +76,7 @@ struct BatchSys {
     int32_t ntiles;
     int32_t method;
     int32_t solo;                 // 1: the iteration SpMV is the single-system kernel (large matrix)
+    int32_t resident;             // CTAs that iterate on it in their shared memory (0: the batch's kernels do)
 };
 
 struct BatchScal {
@@ -81,7 +86,7 @@ struct BatchScal {
     int64_t iter, maxiter;
     int32_t flag, stop, replace, restart;
     int32_t ticket, fresh;        // items of the running kernel finished; BiCGSTAB p = r next
-    int32_t restarts, pad;
+    int32_t restarts, resident;   // iterated by k_batch_resident
     int64_t replacements;
     double true_rr;               // r.r of the last FP64 true residual
 };
@@ -99,8 +104,8 @@ constexpr int kGroups = 6;  // (method, block size): group = 3 * method + block 
 // d_ranges: [0, 8) first matrix item of each group then the end; [8, 16) the same for vector items
 constexpr int kVR = 8;
 // [16, 16 + kGroups): end of each group's matrix items that the iteration SpMV
-// kernels take (the items of systems with their own SpMV follow, for the
-// verification pass only)
+// kernels take (the items of resident systems and of systems with their own SpMV
+// follow, for the verification pass only)
 constexpr int kRanges = 3 * kVR;
 // A system whose FP64 matrix holds at least this many bytes runs its iteration
 // SpMV as one launch of the single-system kernel (autotuned for its matrix, fused
@@ -117,6 +122,7 @@ struct yg_batch_t {
     std::vector<int32_t> used;          // slot in use
     std::vector<yg_matrix> mats;
     std::vector<yg_solve_opts> opts;
+    std::vector<int64_t> nnzb;
     BatchSys *d_sys = nullptr;
     BatchScal *d_scal = nullptr;
     BatchMItem *d_mitems = nullptr;
@@ -130,7 +136,7 @@ struct yg_batch_t {
     int32_t tiles_per_item[4] = {0, 4, 4, 4};
     int32_t lanes[4] = {4, 4, 8, 16};
     int32_t variant[4] = {1, 1, 1, 0};   // SpMV variant per block size: 0 staged, 1 direct
-    unsigned groups_present = 0, graph_groups = 0;
+    unsigned groups_present = 0, graph_groups = 0;  // bits g: systems of group g; bits 8 + g: ones not resident
     bool dirty = false;                 // work tables out of date (systems added, removed or reset)
     int32_t live_items = 0;             // vector items of systems that may still iterate (host view)
     int m = 16;
@@ -181,11 +187,12 @@ enum { SP_CG = 0, SP_VERIFY = 1, SP_BICG_V = 2, SP_BICG_T = 3 };
 
 // ---------------------------------------------------------------- device helpers
 
-enum { ACT_ITER = 0, ACT_VERIFY = 1, ACT_RESTART = 2 };
+enum { ACT_ITER = 0, ACT_VERIFY = 1, ACT_RESTART = 2, ACT_RESIDENT = 3 };
 __device__ __forceinline__ int activity(const BatchScal *sc, int kind) {
     const volatile BatchScal *v = sc;
     const int flag = v->flag, stop = v->stop, rep = v->replace, rst = v->restart;
-    if (kind == ACT_ITER) return flag == BF_RUN && stop == BS_NONE;
+    if (kind == ACT_ITER) return flag == BF_RUN && stop == BS_NONE && !v->resident;
+    if (kind == ACT_RESIDENT) return flag == BF_RUN && stop == BS_NONE;
     if (kind == ACT_VERIFY) return (flag == BF_INIT) || (flag == BF_RUN && (stop == BS_CONV || rep));
     return rst != 0;
 }
@@ -1205,6 +1212,90 @@ __global__ void k_batch_jacobi(int64_t nbrows, int B, const int32_t *__restrict_
     }
 }
 
+// ---------------------------------------------------------------- resident systems
+//
+// An iteration of the kernels above is four launches (PCG, two block sizes) whatever the systems' sizes, each
+// of which waits for the slowest of them.  A PCG system whose matrix fits the shared
+// memory of some CTAs is iterated by one cooperative kernel instead: it has its own
+// group of CTAs, which hold its matrix and vectors and iterate for a block (m
+// iterations; to its end when nobody looks at the systems in between) or until it
+// stops; a mixed-precision residual is replaced on the way.  The verification pass then decides as
+// after a block.  A CTA takes the systems of its queue in the order in which the host
+// placed them, the same order in all queues, so the first system that is not done
+// always has all its CTAs.  A group's size follows from the system alone and a block's
+// end changes no bit of its iterates, so its result does not depend on the others.
+// Measured, before -> now: 24 systems of 1,000 to 40,000 unknowns of 2D problems, FP64,
+// 95 -> 51 ms, mixed 110 -> 62; 14 of up to 20,000: 44 -> 13; 8 of up to 10,000: 21.6 ->
+// 6.7; 3 of up to 4,000: 7.7 -> 2.9.  The trips through L2 of the sums and the gathers
+// bound it; the largest batch also waits for its largest system (27 ms alone).
+struct BatchResident {
+    resident::System m;
+    int32_t sys, blocks;  // slot; CTAs of the group
+};
+
+constexpr int kResCtas = 1;       // CTAs per SM (two of 128 threads: 51.0 ms where one of 256 takes 47.9)
+constexpr int kResThreads = 256;  // 254 registers, no spills (384: 59.1 ms, 512: 92)
+constexpr int kResCheck = 16;     // iterations between looks at a due replacement
+constexpr int kResQueue = 8;      // systems per CTA and launch: bounds what a CTA waits for another
+constexpr int kResJobs = 256;     // systems per launch
+
+// (the system's description and state stay in shared memory: in registers they would
+// leave the gathers too few)
+template <int B, typename VT>
+__device__ __forceinline__ int resident_run(const BatchResident &j, int rank, resident::State &st, unsigned char *smem) {
+    return resident::pcg_run<B, VT, true>(j.m, rank, j.blocks, st, smem);
+}
+
+__global__ void __launch_bounds__(kResThreads, kResCtas)
+k_batch_resident(const BatchResident *__restrict__ jobs, const int2 *__restrict__ queue,  // (system, rank)
+                 const int32_t *__restrict__ begin, const BatchSys *__restrict__ sys, BatchScal *scal, int max_its, int32_t *err) {
+    extern __shared__ __align__(16) unsigned char res_smem[];
+    __shared__ BatchResident j;
+    __shared__ resident::State st;
+    for (int k = begin[blockIdx.x]; k < begin[blockIdx.x + 1]; ++k) {
+        __syncthreads();  // the job before is done with the shared memory
+        const int2 entry = queue[k];
+        if (threadIdx.x == 0) j = jobs[entry.x];
+        __syncthreads();
+        // no CTA changes the state before the last of the group has passed its first sum
+        BatchScal &sc = scal[j.sys];
+        if (!activity(&sc, ACT_RESIDENT)) continue;
+        const int rank = entry.y, B = sys[j.sys].block;
+        const bool f32 = sys[j.sys].precision == YG_PREC_MIXED;
+        if (threadIdx.x == 0)
+            st = resident::State{sc.tol,  sc.bb,    0.0,  sc.maxiter, YG_CRIT_RELRES, max_its, kResCheck, f32 ? 1e-2 * sc.rr_last : 0.0,
+                                 sys[j.sys].val, sys[j.sys].b, 0, sc.iter, sc.rz[0], sc.rr, false};
+        __syncthreads();
+        int flag;
+        if (f32)
+            flag = B == 1   ? resident_run<1, float>(j, rank, st, res_smem)
+                   : B == 2 ? resident_run<2, float>(j, rank, st, res_smem)
+                            : resident_run<3, float>(j, rank, st, res_smem);
+        else
+            flag = B == 1   ? resident_run<1, double>(j, rank, st, res_smem)
+                   : B == 2 ? resident_run<2, double>(j, rank, st, res_smem)
+                            : resident_run<3, double>(j, rank, st, res_smem);
+        if (threadIdx.x == 0 && rank == 0) {
+            sc.rz[0] = sc.rz[1] = st.rz;
+            sc.rr = st.rr;
+            sc.iter = st.iter;
+            sc.stop = flag == resident::FLAG_CONVERGED   ? BS_CONV
+                      : flag == resident::FLAG_BREAKDOWN ? BS_BREAK
+                      : flag == resident::FLAG_NAN       ? BS_NAN
+                      : flag == resident::FLAG_MAXITER   ? BS_MAXIT
+                                                         : BS_NONE;
+            if (st.replaced) {
+                sc.replacements += st.replaced;
+                sc.rr_last = 1e2 * st.rr_replace;
+            }
+        }
+        if (st.timed_out) {
+            if (threadIdx.x == 0) atomicExch(err, (int32_t)YG_TIMEOUT);
+            return;
+        }
+    }
+}
+
 // ---------------------------------------------------------------- host
 
 static int batch_grid(yg_context ctx) { return ctx->num_sms * 4; }
@@ -1300,7 +1391,8 @@ static void prepare_spmv_b(yg_context ctx) {
 }
 
 static bool has(yg_batch bt, int g) { return (bt->groups_present >> g) & 1u; }
-static bool has_bicg(yg_batch bt) { return (bt->groups_present >> 3) != 0; }
+static bool iterates(yg_batch bt, int g) { return (bt->groups_present >> (8 + g)) & 1u; }  // in the batch's kernels
+static bool has_bicg(yg_batch bt) { return (bt->groups_present >> (8 + 3)) != 0; }
 
 // the verification pass (also initialises newly added systems)
 static void launch_verify(yg_batch bt) {
@@ -1362,14 +1454,14 @@ static void launch_iteration(yg_batch bt, int parity) {
         YG_LAUNCHED(ctx);
     }
     for (int g = 0; g < kGroups; ++g)
-        if (has(bt, g)) launch_spmv(bt, g < 3 ? SP_CG : SP_BICG_V, g, parity, 1);
+        if (iterates(bt, g)) launch_spmv(bt, g < 3 ? SP_CG : SP_BICG_V, g, parity, 1);
     launch_solo(bt, SP_CG, parity);
     launch_solo(bt, SP_BICG_V, parity);
     k_batch_v2<<<grid, kThreads, 0, ctx->stream>>>(bt->d_vitems, bt->d_ranges, bt->d_sys, bt->d_scal, parity,
                                                   bt->d_vpart);
     YG_LAUNCHED(ctx);
     for (int g = 3; g < kGroups; ++g)
-        if (has(bt, g)) launch_spmv(bt, SP_BICG_T, g, parity, 1);
+        if (iterates(bt, g)) launch_spmv(bt, SP_BICG_T, g, parity, 1);
     launch_solo(bt, SP_BICG_T, parity);
     k_batch_v3<<<grid, kThreads, 0, ctx->stream>>>(bt->d_vitems, bt->d_ranges, bt->d_sys, bt->d_scal, bt->d_vpart);
     YG_LAUNCHED(ctx);
@@ -1430,9 +1522,10 @@ static yg_status rebuild_items(yg_batch bt) {
         if (pass == 1) ranges[2 * kVR + g] = (int32_t)mitems.size();
         for (int s = 0; s < bt->capacity; ++s) {
             if (!bt->used[s] || bt->sys[s].block != B || bt->sys[s].method != method) continue;
-            if (bt->sys[s].solo != pass) continue;
-            if (pass == 1 && sys_live(bt, s)) solo.push_back({s, bt->mats[s]});
+            if ((bt->sys[s].solo || bt->sys[s].resident) != (pass == 1)) continue;
+            if (bt->sys[s].solo && sys_live(bt, s)) solo.push_back({s, bt->mats[s]});
             present |= 1u << g;
+            if (!bt->sys[s].resident) present |= 1u << (8 + g);
             BatchSys &d = bt->sys[s];
             d.mitem_begin = (int32_t)mitems.size();
             d.vitem_begin = (int32_t)vitems.size();
@@ -1478,6 +1571,142 @@ static yg_status rebuild_items(yg_batch bt) {
     bt->solo = solo;
     bt->live_items = (int32_t)vitems.size();
     bt->dirty = false;
+    return YG_OK;
+}
+
+// Shared memory of a CTA of k_batch_resident: an SM's, less what the runtime and the
+// static arrays take.
+static int64_t resident_room(yg_context ctx) {
+    int sm = 0;
+    cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx->device);
+    return std::min(sm / kResCtas - 4096, (int)ctx->smem_optin - 4096);
+}
+
+// The CTAs a system's resident iterations take; 0 if it does not run resident: its share
+// must fit a CTA's shared memory.  Of a batch that more than fills the GPU the fewest CTAs
+// give the most (a CTA's time in the sums is time another system could use), of one that
+// does not, about the number a system alone would take (pcg_resident.cu).  0.4 of that
+// number lies between: 24 systems of 1,000 to 40,000 unknowns take 47.9 ms with 0.3 of it,
+// 51.1 with 0.4, 60.4 with 0.5 and 62.7 with 0.6; 8 of up to 10,000 take 7.4, 6.7, 6.2 and
+// 5.9; 3 of up to 40,000 take 15.1, 13.8, 12.1 and 11.0.
+static int resident_ctas(yg_context ctx, const BatchSys &d, int64_t nnzb, int64_t row_max) {
+    if (d.method != BM_CG || d.solo || d.nbrows < 1 || d.nbrows >= (1 << 24)) return 0;
+    const int64_t room = resident_room(ctx);
+    int64_t bc, rc;
+    resident::costs(d.block, d.precision == YG_PREC_MIXED, d.corr32 != nullptr, true, &bc, &rc);
+    const int64_t total = nnzb * bc + d.nbrows * rc;
+    const int most = std::min(kResCtas * ctx->num_sms, d.nbrows);
+    int64_t G = (int64_t)((d.block == 1 ? 0.054 : 0.039) * std::sqrt((double)nnzb * d.block * d.block));
+    G = std::max(G, total / room + 1);
+    while (G < most && resident::share(total, row_max, bc, rc, (int)G) > room) ++G;
+    G = std::min<int64_t>(G, most);
+    return resident::share(total, row_max, bc, rc, (int)G) <= room ? (int)G : 0;
+}
+
+static int resident_grid(yg_context ctx) { return kResCtas * ctx->num_sms; }
+
+// Device memory of a launch's tables, beside a context's fixed ones: sums, systems, queues.
+size_t batch_resident_bytes(yg_context ctx) {
+    const size_t most = (size_t)resident_grid(ctx) * kResQueue;
+    return sizeof(resident::SumSlot) * 2 * most + sizeof(BatchResident) * kResJobs +
+           sizeof(int2) * most + sizeof(int32_t) * (resident_grid(ctx) + 1);
+}
+
+// Launches up to max_its iterations of every live resident system.
+static yg_status launch_resident(yg_batch bt, int max_its) {
+    yg_context ctx = bt->ctx;
+    const int ctas = resident_grid(ctx);
+    const size_t most = (size_t)ctas * kResQueue;
+    auto *d_slots = reinterpret_cast<resident::SumSlot *>(ctx->d_slots);
+    auto *d_jobs = reinterpret_cast<BatchResident *>(d_slots + 2 * most);
+    auto *d_queue = reinterpret_cast<int2 *>(d_jobs + kResJobs);
+    auto *d_begin = reinterpret_cast<int32_t *>(d_queue + most);
+    // (the estimate orders the work, no more: iterations grow with the side of a mesh)
+    auto cost = [&](int s) {
+        const BatchSys &d = bt->sys[s];
+        const double its = std::min((double)max_its, (d.block == 1 ? 6.0 : 14.0) * std::sqrt((double)d.nbrows));
+        return its * (5 + 0.03 * d.resident + 8e-4 * (double)bt->nnzb[s] * d.block / d.resident);
+    };
+    std::vector<int> todo;
+    for (int s = 0; s < bt->capacity; ++s)
+        if (sys_live(bt, s) && bt->sys[s].resident) todo.push_back(s);
+    std::stable_sort(todo.begin(), todo.end(), [&](int a, int b) { return cost(a) > cost(b); });
+    while (!todo.empty()) {
+        // the longest system that the free CTAs can take starts first; when there is none,
+        // on to the next time at which CTAs become free
+        std::vector<BatchResident> jobs;
+        std::vector<std::vector<int2>> queue(ctas);
+        std::vector<double> until(ctas, 0.0);
+        double now = 0;
+        int64_t slots = 0;
+        for (;;) {
+            std::vector<int> free;
+            for (int c = 0; c < ctas; ++c)
+                if (until[c] <= now && queue[c].size() < (size_t)kResQueue) free.push_back(c);
+            size_t k = 0;
+            while (k < todo.size() && bt->sys[todo[k]].resident > (int)free.size()) ++k;
+            if (k == todo.size() || jobs.size() == (size_t)kResJobs) {
+                double next = 1e300;
+                for (int c = 0; c < ctas; ++c)
+                    if (until[c] > now && queue[c].size() < (size_t)kResQueue) next = std::min(next, until[c]);
+                if (todo.empty() || next == 1e300 || jobs.size() == (size_t)kResJobs) break;
+                now = next;
+                continue;
+            }
+            const int s = todo[k];
+            todo.erase(todo.begin() + k);
+            const BatchSys &d = bt->sys[s];
+            const int G = d.resident;
+            for (int i = 0; i < G; ++i) {
+                until[free[i]] = now + cost(s);
+                queue[free[i]].push_back(make_int2((int)jobs.size(), i));
+            }
+            const bool f32 = d.precision == YG_PREC_MIXED;
+            const int64_t nnzb = bt->nnzb[s];
+            BatchResident j{};
+            j.sys = s;
+            j.blocks = G;
+            resident::System &m = j.m;
+            m.nbrows = d.nbrows;
+            m.rowptr = d.rowptr;
+            m.col = d.col;
+            m.val = f32 ? static_cast<const void *>(d.val32) : d.val;
+            m.corr = f32 ? d.corr32 : nullptr;
+            m.dinv = d.dinv;
+            m.x = d.x;
+            m.r = d.r;
+            m.p = d.p;
+            m.z = d.q;
+            m.slots = d_slots + slots;
+            m.stride = G;
+            resident::costs(d.block, f32, m.corr != nullptr, true, &m.block_cost, &m.row_cost);
+            m.total_cost = nnzb * m.block_cost + d.nbrows * m.row_cost;
+            m.lanes = resident::row_lanes(d.block, (double)nnzb / d.nbrows, (d.nbrows + G - 1) / G, kResThreads);
+            slots += 2 * G;
+            jobs.push_back(j);
+        }
+        std::vector<int32_t> begin(1, 0);
+        std::vector<int2> entries;
+        for (int c = 0; c < ctas; ++c) {
+            entries.insert(entries.end(), queue[c].begin(), queue[c].end());
+            begin.push_back((int32_t)entries.size());
+        }
+        YG_CUDA(cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(BatchResident) * jobs.size(), cudaMemcpyHostToDevice, ctx->stream));
+        YG_CUDA(cudaMemcpyAsync(d_queue, entries.data(), sizeof(int2) * entries.size(), cudaMemcpyHostToDevice, ctx->stream));
+        YG_CUDA(cudaMemcpyAsync(d_begin, begin.data(), sizeof(int32_t) * begin.size(), cudaMemcpyHostToDevice, ctx->stream));
+        YG_CUDA(cudaMemsetAsync(d_slots, 0, sizeof(resident::SumSlot) * slots, ctx->stream));
+        const BatchResident *aj = d_jobs;
+        const int2 *aq = d_queue;
+        const int32_t *ab = d_begin;
+        const BatchSys *as = bt->d_sys;
+        BatchScal *asc = bt->d_scal;
+        int32_t *ae = ctx->d_err;
+        void *args[] = {&aj, &aq, &ab, &as, &asc, &max_its, &ae};
+        const void *kern = reinterpret_cast<const void *>(&k_batch_resident);
+        const int room = (int)resident_room(ctx);
+        YG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
+        YG_TRY(launch_cooperative(ctx, kern, ctas, kResThreads, (size_t)room, args));
+    }
     return YG_OK;
 }
 
@@ -1570,6 +1799,7 @@ extern "C" yg_status yg_batch_create(yg_context ctx, int32_t capacity, yg_batch 
     bt->used.assign(capacity, 0);
     bt->mats.assign(capacity, nullptr);
     bt->opts.assign(capacity, yg_solve_opts{});
+    bt->nnzb.assign(capacity, 0);
     yg_status s;
     if ((s = dev_alloc_t(ctx, &bt->d_sys, capacity)) != YG_OK || (s = dev_alloc_t(ctx, &bt->d_scal, capacity)) != YG_OK ||
         (s = dev_alloc_t(ctx, &bt->d_ranges, kRanges)) != YG_OK ||
@@ -1681,6 +1911,9 @@ extern "C" yg_status yg_batch_add(yg_batch bt, yg_matrix A, yg_vector b, yg_vect
     d.ntiles = (int32_t)tl.size() - 1;
     d.solo = bt->solo_bytes > 0 && A->nnzb * (int64_t)A->block * A->block * 8 >= bt->solo_bytes;
     if (d.solo) YG_TRY(spmv_autotune_device(A));  // its own SpMV: tune it now, outside any capture
+    int32_t row_max = 0;
+    for (size_t r = 0; r + 1 < rp.size(); ++r) row_max = std::max(row_max, rp[r + 1] - rp[r]);
+    d.resident = resident_ctas(ctx, d, A->nnzb, row_max);
     const int64_t n = A->rows();
     double *dinv = nullptr;
     int32_t *dtiles = nullptr;
@@ -1718,11 +1951,13 @@ extern "C" yg_status yg_batch_add(yg_batch bt, yg_matrix A, yg_vector b, yg_vect
     sc.flag = BF_INIT;
     sc.tol = o.tol;
     sc.maxiter = o.maxiter > 0 ? o.maxiter : n;
+    sc.resident = d.resident > 0;
     bt->sys[s] = d;
     bt->tiles[s] = std::move(tl);
     bt->used[s] = 1;
     bt->mats[s] = A;
     bt->opts[s] = o;
+    bt->nnzb[s] = A->nnzb;
     YG_CUDA(cudaStreamSynchronize(ctx->stream));
     YG_CUDA(cudaMemcpy(bt->d_scal + s, &sc, sizeof(BatchScal), cudaMemcpyHostToDevice));
     bt->h_scal[s] = sc;
@@ -1755,6 +1990,7 @@ extern "C" yg_status yg_batch_reset(yg_batch bt, int32_t slot) {
         sc.flag = BF_INIT;
         sc.tol = o.tol;
         sc.maxiter = o.maxiter > 0 ? o.maxiter : (int64_t)bt->sys[s].nbrows * bt->sys[s].block;
+        sc.resident = bt->sys[s].resident > 0;
         bt->h_scal[s] = sc;
     }
     YG_CUDA(cudaMemcpy(bt->d_scal + s0, bt->h_scal.data() + s0, sizeof(BatchScal) * (s1 - s0), cudaMemcpyHostToDevice));
@@ -1762,12 +1998,21 @@ extern "C" yg_status yg_batch_reset(yg_batch bt, int32_t slot) {
     return YG_OK;
 }
 
-// Launch one block of iterations (graph replay) and the copy of the system
-// states to the host, without waiting.
-static yg_status batch_launch(yg_batch bt) {
+// Launch one block of iterations (at most max_its of the resident systems; a graph
+// replay for the others), a verification pass and the copy of the system states to the
+// host, without waiting.
+static yg_status batch_launch(yg_batch bt, int max_its) {
     yg_context ctx = bt->ctx;
-    YG_CUDA(cudaGraphLaunch(bt->exec, ctx->stream));
-    ctx->launches += bt->graph_kernels;
+    YG_TRY(launch_resident(bt, max_its));
+    bool others = false;
+    for (int s = 0; s < bt->capacity; ++s) others = others || (sys_live(bt, s) && !bt->sys[s].resident);
+    if (others) {
+        if (!bt->exec || bt->graph_groups != bt->groups_present || bt->graph_solo != bt->solo) YG_TRY(capture_graph(bt));
+        YG_CUDA(cudaGraphLaunch(bt->exec, ctx->stream));
+        ctx->launches += bt->graph_kernels;
+    } else {
+        launch_verify(bt);
+    }
     YG_CUDA(cudaMemcpyAsync(bt->h_scal.data(), bt->d_scal, sizeof(BatchScal) * bt->capacity, cudaMemcpyDeviceToHost,
                             ctx->stream));
     YG_CUDA(cudaEventRecord(bt->done, ctx->stream));
@@ -1797,7 +2042,6 @@ static yg_status batch_collect(yg_batch bt, int *active_out) {
 
 static yg_status batch_prepare(yg_batch bt) {
     if (bt->dirty) YG_TRY(rebuild_items(bt));
-    if (!bt->exec || bt->graph_groups != bt->groups_present || bt->graph_solo != bt->solo) YG_TRY(capture_graph(bt));
     launch_verify(bt);  // initialise systems added since the last run
     return YG_OK;
 }
@@ -1810,7 +2054,7 @@ extern "C" yg_status yg_batch_run(yg_batch bt, int32_t max_blocks, int32_t *n_ac
     YG_TRY(batch_prepare(bt));
     int active = 0;
     for (int blk = 0; max_blocks <= 0 || blk < max_blocks; ++blk) {
-        YG_TRY(batch_launch(bt));
+        YG_TRY(batch_launch(bt, max_blocks <= 0 ? 1 << 12 : bt->m));  // (0: nobody looks at the systems in between)
         YG_TRY(batch_collect(bt, &active));
         if (active == 0) break;
     }
@@ -1821,7 +2065,7 @@ extern "C" yg_status yg_batch_run(yg_batch bt, int32_t max_blocks, int32_t *n_ac
 extern "C" yg_status yg_batch_launch(yg_batch bt) {
     if (!bt) return fail(YG_BAD_ARG, "yg_batch_launch: NULL batch");
     YG_TRY(batch_prepare(bt));
-    return batch_launch(bt);
+    return batch_launch(bt, bt->m);
 }
 
 extern "C" yg_status yg_batch_wait(yg_batch bt, int32_t *n_active) {
@@ -1861,7 +2105,7 @@ extern "C" yg_status yg_batch_tune(yg_batch bt) {
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     for (int B = 1; B <= 3; ++B) {
-        const bool cg = has(bt, B - 1), bi = has(bt, 3 + B - 1);
+        const bool cg = iterates(bt, B - 1), bi = iterates(bt, 3 + B - 1);
         if (!cg && !bi) continue;
         float best = 1e30f;
         int bestL = bt->lanes[B], bestT = bt->tiles_per_item[B], bestV = bt->variant[B];

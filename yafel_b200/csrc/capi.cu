@@ -322,10 +322,15 @@ extern "C" yg_status yg_context_create(int32_t device, uint64_t hbm_budget_bytes
     YG_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     yg_status s;
     if ((s = dev_alloc_t(ctx, &ctx->d_partials, 8 * kMaxReduceBlocks)) != YG_OK ||
-        (s = dev_alloc_t(ctx, &ctx->d_scalars, 4)) != YG_OK || (s = dev_alloc_t(ctx, &ctx->d_err, 4)) != YG_OK ||
-        (s = dev_alloc(ctx, &ctx->d_slots, 2 * 32 * 256)) != YG_OK) {
+        (s = dev_alloc_t(ctx, &ctx->d_scalars, 4)) != YG_OK || (s = dev_alloc_t(ctx, &ctx->d_err, 4)) != YG_OK) {
         yg_context_destroy(ctx);
         return s;
+    }
+    // (not counted against the budget, as the pinned block below)
+    if (cudaMalloc(&ctx->d_slots, std::max<size_t>(2 * 32 * 256, batch_resident_bytes(ctx))) != cudaSuccess) {
+        cudaGetLastError();
+        yg_context_destroy(ctx);
+        return fail(YG_OUT_OF_MEMORY, "yg_context_create: no memory for the tables of the cooperative kernels");
     }
     cudaMemset(ctx->d_err, 0, sizeof(int32_t));
     e = cudaMallocHost(&ctx->h_pinned, 64 * sizeof(double));
@@ -344,6 +349,7 @@ extern "C" yg_status yg_context_destroy(yg_context ctx) {
     flush_alloc_cache(ctx);
     for (auto &kv : ctx->allocs) cudaFree(kv.first);
     ctx->allocs.clear();
+    if (ctx->d_slots) cudaFree(ctx->d_slots);
     if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;

@@ -85,7 +85,8 @@ struct yg_context_t {
     double *h_pinned = nullptr;     // 64 doubles of pinned host memory
     KrylovScalars *d_scalars = nullptr;
     int32_t *d_err = nullptr;       // device-side error word (bounded waits that expired)
-    void *d_slots = nullptr;        // grid-wide sums of the cooperative kernels: 2 x 32 bytes per block, 256 blocks
+    void *d_slots = nullptr;        // grid-wide sums of the cooperative kernels (2 x 32 bytes per block, 256
+                                    // blocks), or the sums, systems and queues of a batch's (batch_resident_bytes)
     int reduce_blocks = 592;        // persistent grid for fused Krylov kernels
 };
 
@@ -152,6 +153,7 @@ struct yg_precond_t {
 
 namespace yg {
 
+size_t batch_resident_bytes(yg_context ctx);
 yg_status dev_alloc(yg_context ctx, void **p, size_t bytes);
 void dev_free(yg_context ctx, void *p);
 template <typename T>
