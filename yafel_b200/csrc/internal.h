@@ -84,7 +84,7 @@ struct yg_context_t {
     double *d_partials = nullptr;   // 8 * kMaxReduceBlocks doubles
     double *h_pinned = nullptr;     // 64 doubles of pinned host memory
     KrylovScalars *d_scalars = nullptr;
-    int32_t *d_err = nullptr;       // device-side error word (bounded waits that expired)
+    int32_t *d_err = nullptr;       // error word in pinned host memory (bounded waits that expired)
     void *d_slots = nullptr;        // grid-wide sums of the cooperative kernels (2 x 32 bytes per block, 256
                                     // blocks), or the sums, systems and queues of a batch's (batch_resident_bytes)
     int reduce_blocks = 592;        // persistent grid for fused Krylov kernels
