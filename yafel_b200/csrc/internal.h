@@ -54,7 +54,8 @@ struct KrylovScalars {
     int32_t flag;     // 0 running, 1 converged, 2 breakdown, 3 nan, 4 iteration cap
     int32_t criterion;
     int32_t check_freq;  // BiCGSTAB reference criterion: true-residual check period
-    int32_t pad;
+    int32_t replaced;    // CG, resident: residual replacements of the launch
+    double rr_replace;   // CG, resident: r.r below which the next one is due
     int64_t iter_seen;   // CG: iter as the update kernel saw it (read by the next kernel,
                          // which increments iter: no block reads a value another block writes)
 };
@@ -192,8 +193,8 @@ yg_status matrix_row_extent(yg_matrix A);
 // PCG iterations in one cooperative kernel (pcg_resident.cu)
 yg_status launch_cooperative(yg_context ctx, const void *kern, int grid, int threads, size_t smem, void **args);
 yg_status pcg_resident_fits(yg_matrix A, bool f32, bool jacobi, bool *fits);
-yg_status pcg_resident_launch(yg_matrix A, bool f32, const double *dinv, double *x, double *r, double *p, double *zp,
-                              int max_its, int check, double rr_replace);
+yg_status pcg_resident_launch(yg_matrix A, bool f32, const double *dinv, const double *b, double *x, double *r,
+                              double *p, double *zp, int max_its, int check, double rr_replace);
 // batch engine, host side (batch.cu)
 bool batch_slot_running(yg_batch bt, int32_t slot);
 void batch_slot_stats(yg_batch bt, int32_t slot, yg_solve_stats *out);

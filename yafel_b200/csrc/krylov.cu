@@ -518,7 +518,7 @@ static yg_status pcg_core(yg_matrix A, yg_precond M, const double *b, double *x,
         for (;;) {
             int64_t before = hs.iter;
             if (w.zp) {
-                YG_TRY(pcg_resident_launch(A, f32, dinv, x, w.r, w.p, w.zp, 1 << 12, check_every,
+                YG_TRY(pcg_resident_launch(A, f32, dinv, b, x, w.r, w.p, w.zp, 1 << 12, check_every,
                                            reliable ? 1e-2 * rr_last : 0.0));
             } else if (before < direct_its) {
                 for (int it = 0; it < check_every && before + it < maxiter; ++it) YG_TRY(one(it & 1));
@@ -530,10 +530,14 @@ static yg_status pcg_core(yg_matrix A, yg_precond M, const double *b, double *x,
             }
             YG_TRY(read_scalars(ctx, &hs));
             if (w.zp && hs.flag == FLAG_NAN) YG_TRY(check_device_error(ctx));  // or a grid-wide sum that timed out
+            if (w.zp && hs.replaced) {
+                rr_last = 1e2 * hs.rr_replace;
+                if (replacements) *replacements += hs.replaced;
+            }
             if (prof) YG_TRY(prof->collect(hs.iter - before));
             if (hs.flag == FLAG_RUN) {
                 // replace once the recursive residual fell 10x since the last time
-                if (reliable && hs.rr < 1e-2 * rr_last) {
+                if (reliable && !w.zp && hs.rr < 1e-2 * rr_last) {
                     YG_TRY(replace(0));
                     YG_TRY(read_scalars(ctx, &hs));
                     rr_last = hs.rr;

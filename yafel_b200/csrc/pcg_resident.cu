@@ -26,6 +26,8 @@
 // 30,258 unknowns of order-2 plane elasticity 15.8 -> 9.0; 10,125 unknowns of Q2
 // elasticity 17 -> 11.8.  The trips through L2 of the two sums bound it: a matrix
 // this size takes 1-4 us from shared memory.
+// A mixed-precision solve replaces its residual inside the kernel too (4,225 unknowns:
+// 1.97 -> 1.66 ms a solve of 295 iterations and 8 replacements).
 // Polls are bounded: a block that gives up records YG_TIMEOUT and returns, and so
 // do the others.
 #include "resident.cuh"
@@ -44,6 +46,7 @@ struct ResidentArgs {
     int32_t *err;
     int max_its, check;
     double rr_replace;
+    const double *val64, *b;  // what a residual is replaced from
 };
 
 template <int B, typename VT>
@@ -51,7 +54,7 @@ __global__ void __launch_bounds__(512, 1) k_pcg_resident(ResidentArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     KrylovScalars *S = a.S;
     if (read_flag(&S->flag)) return;  // set before the launch: the same for every block
-    State st{S->tol, S->bb, S->rz0, S->maxiter, S->criterion, a.max_its, a.check, a.rr_replace, nullptr, nullptr, 0, S->iter, S->rz[0], S->rr, false};
+    State st{S->tol, S->bb, S->rz0, S->maxiter, S->criterion, a.max_its, a.check, a.rr_replace, a.val64, a.b, 0, S->iter, S->rz[0], S->rr, false};
     const int flag = pcg_run<B, VT, false>(a.sys, blockIdx.x, gridDim.x, st, smem);
     if (threadIdx.x == 0) {
         if (st.timed_out) atomicExch(a.err, (int32_t)YG_TIMEOUT);
@@ -59,6 +62,8 @@ __global__ void __launch_bounds__(512, 1) k_pcg_resident(ResidentArgs a) {
             S->rz[0] = S->rz[1] = st.rz;
             S->rr = st.rr;
             S->iter = S->iter_seen = st.iter;
+            S->replaced = st.replaced;
+            S->rr_replace = st.rr_replace;
             S->flag = flag;
         }
     }
@@ -116,7 +121,7 @@ static int resident_blocks(yg_matrix A, bool f32, bool jacobi) {
     const double entries = (double)A->nnzb * A->block * A->block;
     const int most = (int)std::min<int64_t>(ctx->num_sms, A->nbrows);
     int G = (int)std::max(16.0, (A->block == 1 ? 0.136 : 0.098) * std::sqrt(entries));
-    while (G < most && resident_smem(A, f32, jacobi, G) > (int64_t)ctx->smem_optin - 2048) G += 4;
+    while (G < most && resident_smem(A, f32, jacobi, G) > (int64_t)ctx->smem_optin - 3072) G += 4;
     return std::min(G, most);
 }
 
@@ -128,7 +133,7 @@ yg_status pcg_resident_fits(yg_matrix A, bool f32, bool jacobi, bool *fits) {
     if (A->block > 3 || A->nbrows < 1 || A->nbrows >= (1 << 24) || ctx->num_sms > kMaxSumBlocks) return YG_OK;
     int64_t bc, rc;
     resident_costs(A, f32, jacobi, &bc, &rc);
-    const int64_t total = A->nnzb * bc + A->nbrows * rc, room = (int64_t)ctx->smem_optin - 2048;
+    const int64_t total = A->nnzb * bc + A->nbrows * rc, room = (int64_t)ctx->smem_optin - 3072;
     if (total / ctx->num_sms > room) return YG_OK;
     YG_TRY(matrix_row_extent(A));
     *fits = resident_smem(A, f32, jacobi, resident_blocks(A, f32, jacobi)) <= room;
@@ -137,8 +142,8 @@ yg_status pcg_resident_fits(yg_matrix A, bool f32, bool jacobi, bool *fits) {
 
 // One launch of at most max_its iterations on the state pcg_core keeps (x, r, p and
 // the scalars; zp: 2 n doubles of scratch).
-yg_status pcg_resident_launch(yg_matrix A, bool f32, const double *dinv, double *x, double *r, double *p, double *zp,
-                              int max_its, int check, double rr_replace) {
+yg_status pcg_resident_launch(yg_matrix A, bool f32, const double *dinv, const double *b, double *x, double *r,
+                              double *p, double *zp, int max_its, int check, double rr_replace) {
     yg_context ctx = A->ctx;
     ResidentArgs a;
     System &m = a.sys;
@@ -162,6 +167,8 @@ yg_status pcg_resident_launch(yg_matrix A, bool f32, const double *dinv, double 
     a.max_its = max_its;
     a.check = check;
     a.rr_replace = rr_replace;
+    a.val64 = A->d_val;
+    a.b = b;
     const int G = resident_blocks(A, f32, dinv != nullptr);
     const double mean = (double)A->nnzb / A->nbrows;
     const int64_t rows = (A->nbrows + G - 1) / G;

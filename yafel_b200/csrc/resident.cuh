@@ -45,9 +45,9 @@ struct State {
     int64_t maxiter;
     int criterion;
     int max_its, check;      // iterations at most; residual replacement is looked at every `check`
-    double rr_replace;       // leave when r.r < rr_replace at such a point (0: never), or, given the
-    const double *val64, *b; // FP64 values and the right-hand side, replace there and go on
-    int replaced;            // how often; then rr_replace follows the residual
+    double rr_replace;       // replace r by b - A x when r.r < rr_replace at such a point (0: never; FP32 values only)
+    const double *val64, *b; // from these
+    int replaced;            // how often; rr_replace follows the residual
     int64_t iter;            // these three are updated
     double rz, rr;
     bool timed_out;
@@ -158,7 +158,8 @@ __device__ inline int first_row(const int32_t *rowptr, int n, int64_t block_cost
 }
 
 // Iterations of one system by CTA `rank` of the group's G (the same state in all of
-// them); x, r and, when the flag returned is FLAG_RUN, p are written back.
+// them; S is one for all threads or one for each, read before the first sum and written
+// after the last); x, r and, when the flag returned is FLAG_RUN, p are written back.
 template <int B, typename VT, bool SPLIT>
 __device__ __forceinline__ int pcg_run(const System &a, int rank, int G, State &S, unsigned char *smem) {
     constexpr int B2 = B * B;
@@ -210,7 +211,8 @@ __device__ __forceinline__ int pcg_run(const System &a, int rank, int G, State &
     }
     const double tol = S.tol, bb = S.bb, rz0 = S.rz0;
     int64_t iter = S.iter;
-    double rz = S.rz, rr = S.rr, beta = 0;
+    double rz = S.rz, rr = S.rr, beta = 0, rr_replace = S.rr_replace;
+    int replaced = 0;
     unsigned epoch = 1;
     int flag = FLAG_RUN;
     double t0, t1;
@@ -306,8 +308,8 @@ __device__ __forceinline__ int pcg_run(const System &a, int rank, int G, State &
         beta = rz_new / rz;
         rz = rz_new;
         // (a slot is written again only after a sum in the other half: all have read it)
-        const bool due = flag == FLAG_RUN && (it + 1) % S.check == 0 && rr < S.rr_replace;
-        if (SPLIT && sizeof(VT) == 4 && due) {
+        const bool due = flag == FLAG_RUN && (it + 1) % S.check == 0 && rr < rr_replace;
+        if (sizeof(VT) == 4 && due) {
             // r = b - A x from the FP64 values; the sums keep alternating between the slots
             for (int i = tid; i < nd; i += nt) a.x[(int64_t)r0 * B + i] = x[i];
             ++epoch;
@@ -341,12 +343,10 @@ __device__ __forceinline__ int pcg_run(const System &a, int rank, int G, State &
                 }
             }
             if (!(ok = group_sum<true, false>(a.slots + a.stride, rank, G, epoch, srz, srr, rz, rr))) break;
-            if (tid == 0) {  // (nobody reads these before the next sum)
-                S.rr_replace = 1e-2 * rr;
-                ++S.replaced;
-            }
+            rr_replace = 1e-2 * rr;
+            ++replaced;
             if (it + 1 >= S.max_its) break;
-        } else if (flag != FLAG_RUN || it + 1 >= S.max_its || due) {
+        } else if (flag != FLAG_RUN || it + 1 >= S.max_its) {
             break;
         }
     }
@@ -360,6 +360,8 @@ __device__ __forceinline__ int pcg_run(const System &a, int rank, int G, State &
     S.iter = iter;
     S.rz = rz;
     S.rr = rr;
+    S.rr_replace = rr_replace;
+    S.replaced = replaced;
     S.timed_out = !ok;
     return flag;
 }
