@@ -1224,10 +1224,9 @@ __global__ void k_batch_jacobi(int64_t nbrows, int B, const int32_t *__restrict_
 // placed them, the same order in all queues, so the first system that is not done
 // always has all its CTAs.  A group's size follows from the system alone and a block's
 // end changes no bit of its iterates, so its result does not depend on the others.
-// Measured, before -> now: 24 systems of 1,000 to 40,000 unknowns of 2D problems, FP64,
-// 95 -> 51 ms, mixed 110 -> 62; 14 of up to 20,000: 44 -> 13; 8 of up to 10,000: 21.6 ->
-// 6.7; 3 of up to 4,000: 7.7 -> 2.9.  The trips through L2 of the sums and the gathers
-// bound it; the largest batch also waits for its largest system (27 ms alone).
+// Measured, before -> now: 14 systems of up to 20,000 unknowns of 2D problems 44 -> 13 ms;
+// 8 of up to 10,000: 21.6 -> 6.5; 3 of up to 4,000: 7.7 -> 2.9.  The trips through L2 of
+// the sums and the gathers bound it.
 struct BatchResident {
     resident::System m;
     int32_t sys, blocks;  // slot; CTAs of the group
@@ -1235,6 +1234,12 @@ struct BatchResident {
 
 constexpr int kResCtas = 1;       // CTAs per SM (two of 128 threads: 51.0 ms where one of 256 takes 47.9)
 constexpr int kResThreads = 256;  // 254 registers, no spills (384: 59.1 ms, 512: 92)
+// Systems whose FP64 matrix and vectors fill at most this many CTAs run resident.  Many
+// larger ones keep the shared kernels busy, which then take less of the GPU's time for
+// each: 128 systems of 1,000 to 200,000 unknowns take 1.29 s without the resident kernel,
+// 1.29 with 48, 1.46 with 80 and 1.75 with 148 (24 of up to 40,000: 97 ms, 91, 49, 49;
+// 14 of up to 20,000: 42, 13, 13, 13).
+constexpr int kResMost = 48;
 constexpr int kResCheck = 16;     // iterations between looks at a due replacement
 constexpr int kResQueue = 8;      // systems per CTA and launch: bounds what a CTA waits for another
 constexpr int kResJobs = 256;     // systems per launch
@@ -1586,8 +1591,8 @@ static int64_t resident_room(yg_context ctx) {
 // must fit a CTA's shared memory.  Of a batch that more than fills the GPU the fewest CTAs
 // give the most (a CTA's time in the sums is time another system could use), of one that
 // does not, about the number a system alone would take (pcg_resident.cu).  0.4 of that
-// number lies between: 24 systems of 1,000 to 40,000 unknowns take 47.9 ms with 0.3 of it,
-// 51.1 with 0.4, 60.4 with 0.5 and 62.7 with 0.6; 8 of up to 10,000 take 7.4, 6.7, 6.2 and
+// number lies between: 24 systems of 1,000 to 40,000 unknowns, all resident, take 47.9 ms
+// with 0.3 of it, 51.1 with 0.4, 60.4 with 0.5 and 62.7 with 0.6; 8 of up to 10,000 take 7.4, 6.7, 6.2 and
 // 5.9; 3 of up to 40,000 take 15.1, 13.8, 12.1 and 11.0.
 static int resident_ctas(yg_context ctx, const BatchSys &d, int64_t nnzb, int64_t row_max) {
     if (d.method != BM_CG || d.solo || d.nbrows < 1 || d.nbrows >= (1 << 24)) return 0;
@@ -1595,6 +1600,9 @@ static int resident_ctas(yg_context ctx, const BatchSys &d, int64_t nnzb, int64_
     int64_t bc, rc;
     resident::costs(d.block, d.precision == YG_PREC_MIXED, d.corr32 != nullptr, true, &bc, &rc);
     const int64_t total = nnzb * bc + d.nbrows * rc;
+    int64_t bc64, rc64;
+    resident::costs(d.block, false, false, true, &bc64, &rc64);
+    if (nnzb * bc64 + d.nbrows * rc64 > kResMost * room) return 0;
     const int most = std::min(kResCtas * ctx->num_sms, d.nbrows);
     int64_t G = (int64_t)((d.block == 1 ? 0.054 : 0.039) * std::sqrt((double)nnzb * d.block * d.block));
     G = std::max(G, total / room + 1);
