@@ -789,7 +789,7 @@ static yg_status launch_assemble(yg_context ctx, const ElementGroup &g, yg_dofma
                                  (size_t)w * asm_warp_doubles(nen, nq, NSD, DPN * DPN, PHYS));
     };
     if (g.shaped != reinterpret_cast<const void *>(kern)) {
-        YG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->smem_optin));
+        YG_TRY(allow_all_smem(ctx, reinterpret_cast<const void *>(kern)));
         // warps per CTA: as many resident warps as the SM holds beside the CTAs' tables
         g.warps = g.resident = 0;
         for (int w = 1; w <= kAsmWarps; ++w) {
@@ -1788,7 +1788,7 @@ static yg_status launch_smooth_gradient(yg_context ctx, const ElementGroup &g, y
     if (smem > ctx->smem_optin)
         return fail(YG_UNSUPPORTED, "LocalSmoothingGradient: element (nen %d, nq %d) needs %zu B of shared memory, "
                     "the device allows %zu", nen, nq, smem, ctx->smem_optin);
-    if (smem > 48 * 1024) YG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) YG_TRY(allow_all_smem(ctx, reinterpret_cast<const void *>(kern)));
     for (size_t c = 0; c + 1 < g.color_ptr.size(); ++c) {
         const int n = g.color_ptr[c + 1] - g.color_ptr[c];
         if (n == 0) continue;
@@ -1818,7 +1818,7 @@ static yg_status launch_zz(yg_context ctx, const ElementGroup &g, yg_dofmap d, c
     if (smem > ctx->smem_optin)
         return fail(YG_UNSUPPORTED, "ZZGradientRecovery: element (nen %d, nq %d) needs %zu B of shared memory", nen, nq,
                     smem);
-    if (smem > 48 * 1024) YG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) YG_TRY(allow_all_smem(ctx, reinterpret_cast<const void *>(kern)));
     for (size_t c = 0; c + 1 < g.color_ptr.size(); ++c) {
         const int n = g.color_ptr[c + 1] - g.color_ptr[c];
         if (n == 0) continue;

@@ -229,6 +229,11 @@ yg_status check_device_error(yg_context ctx) {
     return YG_OK;
 }
 
+yg_status allow_all_smem(yg_context ctx, const void *kern, int fixed) {
+    YG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->smem_optin - fixed));
+    return YG_OK;
+}
+
 int stream_grid(yg_context ctx, int64_t n) {
     int64_t g = (n + kThreads - 1) / kThreads;
     int64_t cap = (int64_t)ctx->num_sms * 8;

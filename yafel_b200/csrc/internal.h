@@ -188,6 +188,11 @@ yg_status vector_dot(yg_context ctx, const double *a, const double *b, int64_t n
 yg_status check_device_error(yg_context ctx);
 yg_status matrix_build_diag(yg_matrix A);
 void flush_alloc_cache(yg_context ctx);
+// Lets `kern` take the device's whole opt-in shared memory (less its `fixed` bytes of static
+// arrays).  The limit belongs to the function on the device and is shared by all contexts and
+// threads, so it is the same constant whatever the next launch needs: a launch's own size,
+// set before it, was lowered by another thread's before it ran.
+yg_status allow_all_smem(yg_context ctx, const void *kern, int fixed = 0);
 // Smallest and largest row length of A into row_min / row_max, measured once.
 yg_status matrix_row_extent(yg_matrix A);
 // PCG iterations in one cooperative kernel (pcg_resident.cu)

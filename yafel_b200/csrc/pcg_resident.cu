@@ -39,6 +39,7 @@ namespace yg {
 using namespace resident;
 
 constexpr int kMaxSumBlocks = 256;
+constexpr int kStaticSmem = 3072;  // shared memory left to the kernel's static arrays and the runtime
 
 struct ResidentArgs {
     System sys;
@@ -121,7 +122,7 @@ static int resident_blocks(yg_matrix A, bool f32, bool jacobi) {
     const double entries = (double)A->nnzb * A->block * A->block;
     const int most = (int)std::min<int64_t>(ctx->num_sms, A->nbrows);
     int G = (int)std::max(16.0, (A->block == 1 ? 0.136 : 0.098) * std::sqrt(entries));
-    while (G < most && resident_smem(A, f32, jacobi, G) > (int64_t)ctx->smem_optin - 3072) G += 4;
+    while (G < most && resident_smem(A, f32, jacobi, G) > (int64_t)ctx->smem_optin - kStaticSmem) G += 4;
     return std::min(G, most);
 }
 
@@ -133,7 +134,7 @@ yg_status pcg_resident_fits(yg_matrix A, bool f32, bool jacobi, bool *fits) {
     if (A->block > 3 || A->nbrows < 1 || A->nbrows >= (1 << 24) || ctx->num_sms > kMaxSumBlocks) return YG_OK;
     int64_t bc, rc;
     resident_costs(A, f32, jacobi, &bc, &rc);
-    const int64_t total = A->nnzb * bc + A->nbrows * rc, room = (int64_t)ctx->smem_optin - 3072;
+    const int64_t total = A->nnzb * bc + A->nbrows * rc, room = (int64_t)ctx->smem_optin - kStaticSmem;
     if (total / ctx->num_sms > room) return YG_OK;
     YG_TRY(matrix_row_extent(A));
     *fits = resident_smem(A, f32, jacobi, resident_blocks(A, f32, jacobi)) <= room;
@@ -176,7 +177,7 @@ yg_status pcg_resident_launch(yg_matrix A, bool f32, const double *dinv, const d
     m.lanes = row_lanes(A->block, mean, rows, threads);
     const size_t smem = (size_t)resident_smem(A, f32, dinv != nullptr, G);
     const void *kern = resident_kernel(A->block, f32);
-    YG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    YG_TRY(allow_all_smem(ctx, kern, kStaticSmem));
     YG_CUDA(cudaMemsetAsync(ctx->d_slots, 0, sizeof(SumSlot) * 2 * kMaxSumBlocks, ctx->stream));
     void *args[] = {&a};
     return launch_cooperative(ctx, kern, G, threads, smem, args);

@@ -377,7 +377,7 @@ static yg_status ilu_factor(yg_precond M, int32_t *done, int *zeros) {
     const int smem = 8 * room * warps;
     int nb = (int)A->nbrows;
     auto kern = k_ilu_factor<B>;
-    YG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    YG_TRY(allow_all_smem(ctx, reinterpret_cast<const void *>(kern)));
     void *args[] = {&nb, &M->d_lower_rows, &A->d_rowptr, &A->d_col, &A->d_diag, &M->d_lu, &done, &zeros, &room, &ctx->d_err};
     return launch_cooperative(ctx, reinterpret_cast<const void *>(kern), ctx->num_sms, 32 * warps, (size_t)smem, args);
 }
