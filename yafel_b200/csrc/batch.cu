@@ -77,6 +77,7 @@ struct BatchSys {
     int32_t method;
     int32_t solo;                 // 1: the iteration SpMV is the single-system kernel (large matrix)
     int32_t resident;             // CTAs that iterate on it in their shared memory (0: the batch's kernels do)
+    int32_t row_max;              // blocks of its longest row
 };
 
 struct BatchScal {
@@ -1594,7 +1595,7 @@ static int64_t resident_room(yg_context ctx) {
 // number lies between: 24 systems of 1,000 to 40,000 unknowns, all resident, take 47.9 ms
 // with 0.3 of it, 51.1 with 0.4, 60.4 with 0.5 and 62.7 with 0.6; 8 of up to 10,000 take 7.4, 6.7, 6.2 and
 // 5.9; 3 of up to 40,000 take 15.1, 13.8, 12.1 and 11.0.
-static int resident_ctas(yg_context ctx, const BatchSys &d, int64_t nnzb, int64_t row_max) {
+static int resident_ctas(yg_context ctx, const BatchSys &d, int64_t nnzb) {
     if (d.method != BM_CG || d.solo || d.nbrows < 1 || d.nbrows >= (1 << 24)) return 0;
     const int64_t room = resident_room(ctx);
     int64_t bc, rc;
@@ -1606,9 +1607,12 @@ static int resident_ctas(yg_context ctx, const BatchSys &d, int64_t nnzb, int64_
     const int most = std::min(kResCtas * ctx->num_sms, d.nbrows);
     int64_t G = (int64_t)((d.block == 1 ? 0.054 : 0.039) * std::sqrt((double)nnzb * d.block * d.block));
     G = std::max(G, total / room + 1);
-    while (G < most && resident::share(total, row_max, bc, rc, (int)G) > room) ++G;
+    while (G < most && resident::share(d.block, total, d.row_max, bc, rc, (int)G) > room) ++G;
     G = std::min<int64_t>(G, most);
-    return resident::share(total, row_max, bc, rc, (int)G) <= room ? (int)G : 0;
+    // (a row that fills most of a CTA can ask for many more: four systems of 40,000 unknowns with a
+    // row of 15,000 took 33.6 ms on 125 CTAs each, 19.0 on the shared kernels)
+    if (G > kResMost) return 0;
+    return resident::share(d.block, total, d.row_max, bc, rc, (int)G) <= room ? (int)G : 0;
 }
 
 static int resident_grid(yg_context ctx) { return kResCtas * ctx->num_sms; }
@@ -1690,6 +1694,7 @@ static yg_status launch_resident(yg_batch bt, int max_its) {
             resident::costs(d.block, f32, m.corr != nullptr, true, &m.block_cost, &m.row_cost);
             m.total_cost = nnzb * m.block_cost + d.nbrows * m.row_cost;
             m.lanes = resident::row_lanes(d.block, (double)nnzb / d.nbrows, (d.nbrows + G - 1) / G, kResThreads);
+            m.long_row = resident::long_row(d.block, m.lanes, d.row_max);
             slots += 2 * G;
             jobs.push_back(j);
         }
@@ -1919,9 +1924,8 @@ extern "C" yg_status yg_batch_add(yg_batch bt, yg_matrix A, yg_vector b, yg_vect
     d.ntiles = (int32_t)tl.size() - 1;
     d.solo = bt->solo_bytes > 0 && A->nnzb * (int64_t)A->block * A->block * 8 >= bt->solo_bytes;
     if (d.solo) YG_TRY(spmv_autotune_device(A));  // its own SpMV: tune it now, outside any capture
-    int32_t row_max = 0;
-    for (size_t r = 0; r + 1 < rp.size(); ++r) row_max = std::max(row_max, rp[r + 1] - rp[r]);
-    d.resident = resident_ctas(ctx, d, A->nnzb, row_max);
+    for (size_t r = 0; r + 1 < rp.size(); ++r) d.row_max = std::max(d.row_max, rp[r + 1] - rp[r]);
+    d.resident = resident_ctas(ctx, d, A->nnzb);
     const int64_t n = A->rows();
     double *dinv = nullptr;
     int32_t *dtiles = nullptr;

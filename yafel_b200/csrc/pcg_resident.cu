@@ -108,7 +108,7 @@ static void resident_costs(yg_matrix A, bool f32, bool jacobi, int64_t *block, i
 static int64_t resident_smem(yg_matrix A, bool f32, bool jacobi, int G) {
     int64_t bc, rc;
     resident_costs(A, f32, jacobi, &bc, &rc);
-    return share(A->nnzb * bc + A->nbrows * rc, A->row_max, bc, rc, G);
+    return share(A->block, A->nnzb * bc + A->nbrows * rc, A->row_max, bc, rc, G);
 }
 
 // Blocks of a resident solve, one per SM at most.  The two sums cost 4.5 us + 0.028 us
@@ -175,6 +175,7 @@ yg_status pcg_resident_launch(yg_matrix A, bool f32, const double *dinv, const d
     const int64_t rows = (A->nbrows + G - 1) / G;
     const int threads = rows * (mean > 8 ? 8 : 4) > 512 ? 512 : 256;
     m.lanes = row_lanes(A->block, mean, rows, threads);
+    m.long_row = long_row(A->block, m.lanes, A->row_max);
     const size_t smem = (size_t)resident_smem(A, f32, dinv != nullptr, G);
     const void *kern = resident_kernel(A->block, f32);
     YG_TRY(allow_all_smem(ctx, kern, kStaticSmem));

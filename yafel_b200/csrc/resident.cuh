@@ -7,6 +7,7 @@
 #include "device_common.cuh"
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 
 namespace yg {
@@ -27,6 +28,16 @@ struct alignas(32) SumSlot {
 // and 2, 51.1 with these).
 constexpr int gathers(int B) { return B == 1 ? 8 : (B == 2 ? 4 : 2); }
 
+// A row of more than kLongRounds rounds of its lanes is left to a whole warp: with the
+// 2 lanes that suit a mean of 7 entries, a row of 1,000 took 62 rounds while all others
+// waited (us an iteration, streaming kernels / lanes by the mean / a warp for a long row:
+// 5,000 unknowns with a row of 1,000 21 / 32 / 12, with one of 4,000 34 / 108 / 19; 40,000 with one of
+// 15,000 84 / 406 / 67).
+constexpr int kLongRounds = 4;
+// Long rows of a CTA at most: a row longer than kLongRounds * lanes * gathers(B) blocks fills 512
+// bytes of its shared memory or more.
+constexpr int kLongRows = 512;
+
 struct System {
     int nbrows;
     const int32_t *rowptr, *col;
@@ -39,6 +50,7 @@ struct System {
     int stride;
     int64_t block_cost, row_cost, total_cost;  // shared memory bytes per block, per block row, of all
     int lanes;               // lanes per block row
+    int long_row;            // rows of more blocks are long (INT_MAX: none is)
 };
 struct State {
     double tol, bb, rz0;
@@ -163,8 +175,9 @@ __device__ inline int first_row(const int32_t *rowptr, int n, int64_t block_cost
 template <int B, typename VT, bool SPLIT>
 __device__ __forceinline__ int pcg_run(const System &a, int rank, int G, State &S, unsigned char *smem) {
     constexpr int B2 = B * B;
-    __shared__ int bounds[2];
+    __shared__ int bounds[2], nlong;
     const int tid = threadIdx.x, nt = blockDim.x;
+    if (tid == 0) nlong = 0;
     if (tid < 64) {
         const int64_t t = rank + (tid >> 5);
         const int r = t == G ? a.nbrows : first_row(a.rowptr, a.nbrows, a.block_cost, a.row_cost, t * a.total_cost / G);
@@ -173,7 +186,7 @@ __device__ __forceinline__ int pcg_run(const System &a, int rank, int G, State &
     __syncthreads();
     const int r0 = bounds[0], nr = bounds[1] - r0, nd = nr * B;
     const int e0 = a.rowptr[r0], nb = a.rowptr[bounds[1]] - e0;
-    // shared memory: values | columns | row pointers | x, r, p, q (z after the update), dinv, correction
+    // shared memory: values | columns | row pointers | x, r, p, q (z after the update), dinv, correction | long rows
     auto up = [](size_t v) { return (v + 15) & ~(size_t)15; };
     VT *val = reinterpret_cast<VT *>(smem);
     int32_t *col = reinterpret_cast<int32_t *>(smem + up((size_t)nb * B2 * sizeof(VT)));
@@ -181,6 +194,7 @@ __device__ __forceinline__ int pcg_run(const System &a, int rank, int G, State &
     double *x = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(rp) + up((size_t)(nr + 1) * 4));
     double *r = x + nd, *p = r + nd, *q = p + nd, *dinv = q + nd;
     double *corr = dinv + (a.dinv ? nd : 0);
+    unsigned short *longs = reinterpret_cast<unsigned short *>(corr + (a.corr ? nr * B2 : 0));
     const VT *gval = static_cast<const VT *>(a.val) + (int64_t)e0 * B2;
     for (int i = tid; i < nb * B2; i += nt) val[i] = gval[i];
     for (int i = tid; i < nb; i += nt) col[i] = a.col[e0 + i];
@@ -209,6 +223,19 @@ __device__ __forceinline__ int pcg_run(const System &a, int rank, int G, State &
         q[i] = v;
         publish(i, v, 0.0);
     }
+    if (a.long_row != INT_MAX) {
+        __syncthreads();
+        if (tid < 32) {
+            int n = 0;
+            for (int i0 = 0; i0 < nr; i0 += 32) {
+                const bool is = i0 + tid < nr && rp[i0 + tid + 1] - rp[i0 + tid] > a.long_row;
+                const unsigned m = __ballot_sync(0xffffffffu, is);
+                if (is) longs[n + __popc(m & ((1u << tid) - 1))] = (unsigned short)(i0 + tid);
+                n += __popc(m);
+            }
+            if (tid == 0) nlong = n;
+        }
+    }
     const double tol = S.tol, bb = S.bb, rz0 = S.rz0;
     int64_t iter = S.iter;
     double rz = S.rz, rr = S.rr, beta = 0, rr_replace = S.rr_replace;
@@ -217,66 +244,73 @@ __device__ __forceinline__ int pcg_run(const System &a, int rank, int G, State &
     int flag = FLAG_RUN;
     double t0, t1;
     bool ok = group_sum<false, true>(a.slots + a.stride, rank, G, epoch, 0, 0, t0, t1);
-    const int L = a.lanes, lane = tid & (L - 1), group = tid / L, ngroups = nt / L;
+    // products: `lanes` lanes a row, then a warp for each long row
+    const int passes = a.long_row != INT_MAX ? 2 : 1;
     for (int it = 0; ok; ++it) {
         for (int i = tid; i < nd; i += nt) p[i] = fma(beta, p[i], q[i]);
         __syncthreads();  // p is read and q overwritten by other threads
         double pq = 0;
-        for (int rb = 0; rb < nr; rb += ngroups) {  // the lanes of a warp take the same steps
-            const int row = rb + group;
-            double acc[B];
+        for (int pass = 0; pass < passes; ++pass) {
+            const int L = pass ? 32 : a.lanes, lane = tid & (L - 1), count = pass ? nlong : nr;
+            for (int rb = 0; rb < count; rb += nt / L) {  // the lanes of a warp take the same steps
+                int row = rb + tid / L;
+                bool on = row < count;
+                if (pass && on) row = longs[row];
+                const int js = on ? rp[row] : 0, je = on ? rp[row + 1] : 0;
+                if (!pass) on = on && je - js <= a.long_row;
+                double acc[B];
 #pragma unroll
-            for (int i = 0; i < B; ++i) acc[i] = 0;
-            if (row < nr) {
-                const int je = rp[row + 1];
-                constexpr int U = gathers(B);
-                for (int j0 = rp[row] + lane; j0 < je; j0 += U * L) {
-                    double v[U][2 * B];
+                for (int i = 0; i < B; ++i) acc[i] = 0;
+                if (on) {
+                    constexpr int U = gathers(B);
+                    for (int j0 = js + lane; j0 < je; j0 += U * L) {
+                        double v[U][2 * B];
 #pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        const int j = j0 + u * L;
-                        if (j < je) {
-                            if (!SPLIT || B == 2) {
-                                const double *z = SPLIT ? a.z + (int64_t)col[j] * B : a.zp + (int64_t)col[j] * 2 * B;
-                                const double *p2 = SPLIT ? a.p + (int64_t)col[j] * B : z + B;
+                        for (int u = 0; u < U; ++u) {
+                            const int j = j0 + u * L;
+                            if (j < je) {
+                                if (!SPLIT || B == 2) {
+                                    const double *z = SPLIT ? a.z + (int64_t)col[j] * B : a.zp + (int64_t)col[j] * 2 * B;
+                                    const double *p2 = SPLIT ? a.p + (int64_t)col[j] * B : z + B;
 #pragma unroll
-                                for (int k = 0; k < B; ++k) {
-                                    const double2 d = reinterpret_cast<const double2 *>(SPLIT && k ? p2 : z)[SPLIT ? 0 : k];
-                                    v[u][2 * k] = d.x;
-                                    v[u][2 * k + 1] = d.y;
-                                }
-                            } else {
+                                    for (int k = 0; k < B; ++k) {
+                                        const double2 d = reinterpret_cast<const double2 *>(SPLIT && k ? p2 : z)[SPLIT ? 0 : k];
+                                        v[u][2 * k] = d.x;
+                                        v[u][2 * k + 1] = d.y;
+                                    }
+                                } else {
 #pragma unroll
-                                for (int k = 0; k < B; ++k) {
-                                    v[u][k] = a.z[(int64_t)col[j] * B + k];
-                                    v[u][B + k] = a.p[(int64_t)col[j] * B + k];
+                                    for (int k = 0; k < B; ++k) {
+                                        v[u][k] = a.z[(int64_t)col[j] * B + k];
+                                        v[u][B + k] = a.p[(int64_t)col[j] * B + k];
+                                    }
                                 }
                             }
                         }
-                    }
 #pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        const int j = j0 + u * L;
-                        if (j < je) {
+                        for (int u = 0; u < U; ++u) {
+                            const int j = j0 + u * L;
+                            if (j < je) {
 #pragma unroll
-                            for (int c = 0; c < B; ++c) {
-                                const double pc = fma(beta, v[u][B + c], v[u][c]);
+                                for (int c = 0; c < B; ++c) {
+                                    const double pc = fma(beta, v[u][B + c], v[u][c]);
 #pragma unroll
-                                for (int i = 0; i < B; ++i) acc[i] = fma((double)val[j * B2 + i * B + c], pc, acc[i]);
+                                    for (int i = 0; i < B; ++i) acc[i] = fma((double)val[j * B2 + i * B + c], pc, acc[i]);
+                                }
                             }
                         }
                     }
                 }
-            }
 #pragma unroll
-            for (int i = 0; i < B; ++i)
-                for (int o = L >> 1; o > 0; o >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
-            if (row < nr && lane == 0) {
-                if (a.corr) add_corr<B>(corr, p, row, acc);
+                for (int i = 0; i < B; ++i)
+                    for (int o = L >> 1; o > 0; o >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+                if (on && lane == 0) {
+                    if (a.corr) add_corr<B>(corr, p, row, acc);
 #pragma unroll
-                for (int i = 0; i < B; ++i) {
-                    q[row * B + i] = acc[i];
-                    pq = fma(acc[i], p[row * B + i], pq);
+                    for (int i = 0; i < B; ++i) {
+                        q[row * B + i] = acc[i];
+                        pq = fma(acc[i], p[row * B + i], pq);
+                    }
                 }
             }
         }
@@ -315,30 +349,37 @@ __device__ __forceinline__ int pcg_run(const System &a, int rank, int G, State &
             ++epoch;
             if (!(ok = group_sum<false, true>(a.slots, rank, G, epoch, 0, 0, t0, t1))) break;
             srz = srr = 0;
-            for (int rb = 0; rb < nr; rb += ngroups) {
-                const int row = rb + group;
-                double acc[B];
+            for (int pass = 0; pass < passes; ++pass) {
+                const int L = pass ? 32 : a.lanes, lane = tid & (L - 1), count = pass ? nlong : nr;
+                for (int rb = 0; rb < count; rb += nt / L) {
+                    int row = rb + tid / L;
+                    bool on = row < count;
+                    if (pass && on) row = longs[row];
+                    const int js = on ? rp[row] : 0, je = on ? rp[row + 1] : 0;
+                    if (!pass) on = on && je - js <= a.long_row;
+                    double acc[B];
 #pragma unroll
-                for (int i = 0; i < B; ++i) acc[i] = 0;
-                if (row < nr) {
-                    for (int j = rp[row] + lane; j < rp[row + 1]; j += L) {
-                        const double *v = S.val64 + (int64_t)(e0 + j) * B2, *xc = a.x + (int64_t)col[j] * B;
+                    for (int i = 0; i < B; ++i) acc[i] = 0;
+                    if (on) {
+                        for (int j = js + lane; j < je; j += L) {
+                            const double *v = S.val64 + (int64_t)(e0 + j) * B2, *xc = a.x + (int64_t)col[j] * B;
 #pragma unroll
-                        for (int c = 0; c < B; ++c)
+                            for (int c = 0; c < B; ++c)
 #pragma unroll
-                            for (int i = 0; i < B; ++i) acc[i] = fma(v[i * B + c], xc[c], acc[i]);
+                                for (int i = 0; i < B; ++i) acc[i] = fma(v[i * B + c], xc[c], acc[i]);
+                        }
                     }
-                }
 #pragma unroll
-                for (int i = 0; i < B; ++i)
-                    for (int o = L >> 1; o > 0; o >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
-                if (row < nr && lane == 0) {
+                    for (int i = 0; i < B; ++i)
+                        for (int o = L >> 1; o > 0; o >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+                    if (on && lane == 0) {
 #pragma unroll
-                    for (int i = 0; i < B; ++i) {
-                        const double ri = S.b[(int64_t)(r0 + row) * B + i] - acc[i];
-                        r[row * B + i] = ri;
-                        srz += ri * (a.dinv ? dinv[row * B + i] * ri : ri);
-                        srr += ri * ri;
+                        for (int i = 0; i < B; ++i) {
+                            const double ri = S.b[(int64_t)(r0 + row) * B + i] - acc[i];
+                            r[row * B + i] = ri;
+                            srz += ri * (a.dinv ? dinv[row * B + i] * ri : ri);
+                            srr += ri * ri;
+                        }
                     }
                 }
             }
@@ -373,9 +414,17 @@ inline void costs(int B, bool f32, bool corr, bool jacobi, int64_t *block, int64
     *row = 4 + 8 * B * (jacobi ? 5 : 4) + (corr ? 8 * B * B : 0);
 }
 
-// Shared memory of the largest share among G CTAs: at most the mean and one row more.
-inline int64_t share(int64_t total_cost, int64_t row_max, int64_t block_cost, int64_t row_cost, int G) {
-    return (total_cost + G - 1) / G + row_max * block_cost + row_cost + 256;
+// Shared memory of the largest share among G CTAs: at most the mean and one row more, and
+// the list of long rows where there can be any.
+inline int64_t share(int B, int64_t total_cost, int64_t row_max, int64_t block_cost, int64_t row_cost, int G) {
+    const int64_t list = row_max > kLongRounds * 2 * gathers(B) ? sizeof(unsigned short) * kLongRows : 0;
+    return (total_cost + G - 1) / G + row_max * block_cost + row_cost + 256 + list;
+}
+
+// The row length above which a row takes a warp.
+inline int long_row(int B, int lanes, int64_t row_max) {
+    const int n = kLongRounds * lanes * gathers(B);
+    return lanes < 32 && row_max > n ? n : INT_MAX;
 }
 
 // Lanes per block row: one round of gathers each, more where the threads allow.
