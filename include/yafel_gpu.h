@@ -321,7 +321,9 @@ YG_API yg_status yg_spmv_bench(yg_matrix A, yg_vector x, yg_vector y, int32_t pr
  * substitution with unit L then backward substitution with U). */
 enum { YG_PRECOND_IDENTITY = 0, YG_PRECOND_JACOBI = 1, YG_PRECOND_ILU0 = 2 };
 YG_API yg_status yg_precond_create(yg_matrix A, int32_t kind, yg_precond *out);
-/* M.solve(z) in place (Preconditioner.hpp:9-21). */
+/* M.solve(z) in place (Preconditioner.hpp:9-21).  Asynchronous: an ILU(0) wait
+ * that expired (YG_TIMEOUT) is reported by the next call that waits for the
+ * context, e.g. the download of z. */
 YG_API yg_status yg_precond_apply(yg_precond M, yg_vector z);
 /* Frees M; valid after A has been destroyed (M keeps A's context, not A), but
  * not after that context has been destroyed. */

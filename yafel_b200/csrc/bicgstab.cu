@@ -250,7 +250,7 @@ static yg_status read_s(yg_context ctx, KrylovScalars *out) {
     YG_CUDA(cudaMemcpyAsync(ctx->h_pinned, ctx->d_scalars, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, ctx->stream));
     YG_CUDA(cudaStreamSynchronize(ctx->stream));
     memcpy(out, ctx->h_pinned, sizeof(KrylovScalars));
-    return YG_OK;
+    return check_device_error(ctx);  // a wait that expired ends the solve, whatever the scalars say
 }
 
 struct BGraph {

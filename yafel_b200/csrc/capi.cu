@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>
+#include <cstdlib>
 #include <cstring>
 #include <numeric>
 
@@ -254,7 +255,7 @@ yg_status vector_dot(yg_context ctx, const double *a, const double *b, int64_t n
                             cudaMemcpyDeviceToHost, ctx->stream));
     YG_CUDA(cudaStreamSynchronize(ctx->stream));
     *out = ctx->h_pinned[0];
-    return YG_OK;
+    return check_device_error(ctx);
 }
 
 yg_status matrix_build_diag(yg_matrix A) {
@@ -338,6 +339,7 @@ extern "C" yg_status yg_context_create(int32_t device, uint64_t hbm_budget_bytes
         yg_context_destroy(ctx);
         return fail(YG_OUT_OF_MEMORY, "yg_context_create: no memory for the tables of the cooperative kernels");
     }
+    if (const char *polls = getenv("YAFEL_B200_WAIT_POLLS")) ctx->wait_polls = std::max(0ll, atoll(polls));
     e = cudaMallocHost(&ctx->h_pinned, 64 * sizeof(double));
     if (e == cudaSuccess) e = cudaMallocHost(&ctx->d_err, 64);
     if (e == cudaSuccess) *ctx->d_err = 0;
@@ -434,7 +436,7 @@ extern "C" yg_status yg_vector_download(yg_vector v, double *host, int64_t n) {
     if (!v || (!host && n) || n != v->n) return fail(YG_BAD_ARG, "yg_vector_download: size mismatch");
     YG_CUDA(cudaMemcpyAsync(host, v->d, sizeof(double) * n, cudaMemcpyDeviceToHost, v->ctx->stream));
     YG_CUDA(cudaStreamSynchronize(v->ctx->stream));
-    return YG_OK;
+    return check_device_error(v->ctx);
 }
 
 extern "C" yg_status yg_vector_fill(yg_vector v, double value) {

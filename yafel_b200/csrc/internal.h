@@ -86,6 +86,8 @@ struct yg_context_t {
     double *h_pinned = nullptr;     // 64 doubles of pinned host memory
     KrylovScalars *d_scalars = nullptr;
     int32_t *d_err = nullptr;       // error word in pinned host memory (bounded waits that expired)
+    long long wait_polls = 1ll << 24;  // polls of one wait of an ILU(0) kernel (seconds; a wait takes microseconds);
+                                       // YAFEL_B200_WAIT_POLLS when the context is created: tests let waits expire
     void *d_slots = nullptr;        // grid-wide sums of the cooperative kernels (2 x 32 bytes per block, 256
                                     // blocks), or the sums, systems and queues of a batch's (batch_resident_bytes)
     int reduce_blocks = 592;        // persistent grid for fused Krylov kernels

@@ -321,7 +321,7 @@ static yg_status read_scalars(yg_context ctx, KrylovScalars *out) {
     YG_CUDA(cudaMemcpyAsync(ctx->h_pinned, ctx->d_scalars, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, ctx->stream));
     YG_CUDA(cudaStreamSynchronize(ctx->stream));
     memcpy(out, ctx->h_pinned, sizeof(KrylovScalars));
-    return YG_OK;
+    return check_device_error(ctx);  // a wait that expired ends the solve, whatever the scalars say
 }
 
 static yg_status true_relres(yg_matrix A, const double *b, const double *x, double *tmp, double *out) {
@@ -529,7 +529,6 @@ static yg_status pcg_core(yg_matrix A, yg_precond M, const double *b, double *x,
                 ctx->launches += g.kernels;
             }
             YG_TRY(read_scalars(ctx, &hs));
-            if (w.zp && hs.flag == FLAG_NAN) YG_TRY(check_device_error(ctx));  // or a grid-wide sum that timed out
             if (w.zp && hs.replaced) {
                 rr_last = 1e2 * hs.rr_replace;
                 if (replacements) *replacements += hs.replaced;

@@ -52,7 +52,13 @@ __global__ void k_jacobi_apply(int64_t n, const double *__restrict__ dinv, const
 // row r of them at r * len * B (len blocks); column e of a row is
 // B * col[e / B] + e % B.
 
-constexpr long long kWaitLimit = 1ll << 24;  // polls of one wait (seconds; a wait takes microseconds)
+// A wait of a launch: polls it may take, the launch's own abort word (a warp that gives
+// up sets it and the others follow; the context's error word may still hold an earlier
+// launch's) and the context's error word.
+struct Waits {
+    long long limit;
+    int32_t *abort, *err;
+};
 constexpr unsigned long long kPending = 0x7ff4a11ce0000001ull;  // a signalling NaN: no arithmetic gives it
 
 __device__ __forceinline__ double ld_relaxed(const double *p) {
@@ -72,15 +78,17 @@ __device__ __forceinline__ bool pending(double v) { return (unsigned long long)_
 
 // One more failed poll of a wait: false when the wait gives up (its limit, or
 // another warp's: then the error word is set).
-__device__ __forceinline__ bool wait_on(long long &spins, int32_t *err) {
-    if (++spins > kWaitLimit) {
-        atomicExch(err, (int32_t)YG_TIMEOUT);
+__device__ __forceinline__ bool wait_on(long long &spins, const Waits &w) {
+    if (++spins > w.limit) {
+        atomicExch(w.err, (int32_t)YG_TIMEOUT);
+        atomicExch(w.abort, 1);
         return false;
     }
-    return (spins & 1023) || ld_relaxed_i(err) == 0;
+    return (spins & 1023) || ld_relaxed_i(w.abort) == 0;
 }
 
-__global__ void k_fill_pending(int64_t n, double *__restrict__ z) {
+__global__ void k_fill_pending(int64_t n, double *__restrict__ z, int32_t *__restrict__ abort) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *abort = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         z[i] = __longlong_as_double((long long)kPending);
 }
@@ -116,7 +124,7 @@ template <int B>
 __global__ void __launch_bounds__(kThreads)
 k_ilu_factor(int nbrows, const int32_t *__restrict__ rows, const int32_t *__restrict__ rowptr,
              const int32_t *__restrict__ col, const int32_t *__restrict__ diag, double *lu, int32_t *done,
-             int *__restrict__ zero_pivots, int room, int32_t *err) {
+             int *__restrict__ zero_pivots, int room, Waits waits) {
     extern __shared__ double sm[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nwb = blockDim.x >> 5;
     for (int t = blockIdx.x * nwb + wib; t < nbrows; t += gridDim.x * nwb) {
@@ -141,7 +149,7 @@ k_ilu_factor(int nbrows, const int32_t *__restrict__ rows, const int32_t *__rest
                     const unsigned m = __ballot_sync(0xffffffffu, ok);
                     ready = jj + (m == 0xffffffffu ? 32 : __ffs(~m) - 1);
                     if (ready > jj) break;
-                    if (!__all_sync(0xffffffffu, wait_on(spins, err))) return;
+                    if (!__all_sync(0xffffffffu, wait_on(spins, waits))) return;
                 }
                 asm volatile("fence.acq_rel.gpu;" ::: "memory");
             }
@@ -242,7 +250,7 @@ k_ilu_factor(int nbrows, const int32_t *__restrict__ rows, const int32_t *__rest
 // polled: sums over the warp in every lane.  False when a wait gave up.
 template <int B>
 __device__ __forceinline__ bool row_sums(const int32_t *__restrict__ bc, const double *__restrict__ l, int n, int e0,
-                                         int e1, const double *z, double (&s)[B], int32_t *err) {
+                                         int e1, const double *z, double (&s)[B], const Waits &waits) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int r = 0; r < B; ++r) s[r] = 0;
@@ -270,7 +278,7 @@ __device__ __forceinline__ bool row_sums(const int32_t *__restrict__ bc, const d
 #pragma unroll
             for (int k = 0; k < U; ++k) all = all && !pending(x[k]);
             all = __all_sync(0xffffffffu, all);
-            if (!all && !__all_sync(0xffffffffu, wait_on(spins, err))) return false;
+            if (!all && !__all_sync(0xffffffffu, wait_on(spins, waits))) return false;
         }
 #pragma unroll
         for (int k = 0; k < U; ++k)
@@ -295,7 +303,7 @@ __global__ void __launch_bounds__(kThreads)
 k_ilu_apply(int nbrows, const int32_t *__restrict__ lower, const int32_t *__restrict__ upper,
             const int32_t *__restrict__ rowptr, const int32_t *__restrict__ col, const int32_t *__restrict__ diag,
             const double *__restrict__ lu, const double *rin, double *zf, double *zb, double *z,
-            const int32_t *__restrict__ flag, int32_t *err) {
+            const int32_t *__restrict__ flag, Waits waits) {
     if (flag && read_flag(flag)) return;
     const int lane = threadIdx.x & 31;
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
@@ -311,7 +319,7 @@ k_ilu_apply(int nbrows, const int32_t *__restrict__ lower, const int32_t *__rest
 #pragma unroll
             for (int j = 0; j < r; ++j) d[r][j] = has ? l[r * n + nl * B + j] : 0.0;
         }
-        if (!row_sums<B>(col + b0, l, n, 0, nl * B, zf, s, err)) return;
+        if (!row_sums<B>(col + b0, l, n, 0, nl * B, zf, s, waits)) return;
 #pragma unroll
         for (int r = 0; r < B; ++r) {
             x[r] -= s[r];
@@ -332,10 +340,10 @@ k_ilu_apply(int nbrows, const int32_t *__restrict__ lower, const int32_t *__rest
 #pragma unroll
             for (int j = r; j < B; ++j) d[r][j] = has ? l[r * n + nl * B + j] : (j == r && n > 0 ? l[r * n] : 0.0);
         // (without a diagonal every entry but the first, the divisor, counts)
-        if (!row_sums<B>(col + b0, l, n, has ? (nl + 1) * B : max(nl * B, 1), n, zb, s, err)) return;
+        if (!row_sums<B>(col + b0, l, n, has ? (nl + 1) * B : max(nl * B, 1), n, zb, s, waits)) return;
         if (!has) {
             double f[B];
-            if (!row_sums<B>(col + b0, l, n, 1, nl * B, zf, f, err)) return;
+            if (!row_sums<B>(col + b0, l, n, 1, nl * B, zf, f, waits)) return;
 #pragma unroll
             for (int r = 0; r < B; ++r) s[r] += f[r];
         }
@@ -348,7 +356,7 @@ k_ilu_apply(int nbrows, const int32_t *__restrict__ lower, const int32_t *__rest
                 all = all && !pending(x[r]);
             }
             all = __all_sync(0xffffffffu, all);
-            if (!all && !__all_sync(0xffffffffu, wait_on(spins, err))) return;
+            if (!all && !__all_sync(0xffffffffu, wait_on(spins, waits))) return;
         }
 #pragma unroll
         for (int r = B - 1; r >= 0; --r) {
@@ -365,6 +373,9 @@ k_ilu_apply(int nbrows, const int32_t *__restrict__ lower, const int32_t *__rest
     }
 }
 
+// (d_tmp: the factorization's count of zero pivots, then the abort word)
+static Waits waits_of(yg_precond M) { return {M->ctx->wait_polls, reinterpret_cast<int32_t *>(M->d_tmp) + 1, M->ctx->d_err}; }
+
 template <int B>
 static yg_status ilu_factor(yg_precond M, int32_t *done, int *zeros) {
     yg_matrix A = M->A;
@@ -378,7 +389,8 @@ static yg_status ilu_factor(yg_precond M, int32_t *done, int *zeros) {
     int nb = (int)A->nbrows;
     auto kern = k_ilu_factor<B>;
     YG_TRY(allow_all_smem(ctx, reinterpret_cast<const void *>(kern)));
-    void *args[] = {&nb, &M->d_lower_rows, &A->d_rowptr, &A->d_col, &A->d_diag, &M->d_lu, &done, &zeros, &room, &ctx->d_err};
+    Waits waits = waits_of(M);
+    void *args[] = {&nb, &M->d_lower_rows, &A->d_rowptr, &A->d_col, &A->d_diag, &M->d_lu, &done, &zeros, &room, &waits};
     return launch_cooperative(ctx, reinterpret_cast<const void *>(kern), ctx->num_sms, 32 * warps, (size_t)smem, args);
 }
 
@@ -389,11 +401,12 @@ static yg_status ilu_apply(yg_precond M, const double *r, double *z, const int32
     const int64_t n = A->rows();
     if (n == 0) return YG_OK;
     double *zf = M->d_z, *zb = M->d_z + n;
-    k_fill_pending<<<stream_grid(ctx, 2 * n), kThreads, 0, ctx->stream>>>(2 * n, M->d_z);
+    Waits waits = waits_of(M);
+    k_fill_pending<<<stream_grid(ctx, 2 * n), kThreads, 0, ctx->stream>>>(2 * n, M->d_z, waits.abort);
     YG_LAUNCHED(ctx);
     int nb = (int)A->nbrows;
     void *args[] = {&nb, &M->d_lower_rows, &M->d_upper_rows, &A->d_rowptr, &A->d_col, &A->d_diag, &M->d_lu, &r, &zf, &zb, &z,
-                    &flag, &ctx->d_err};
+                    &flag, &waits};
     const void *kern = nullptr;
     switch (A->block) {
     case 1: kern = reinterpret_cast<const void *>(&k_ilu_apply<1>); break;
@@ -457,7 +470,7 @@ static yg_status build_ilu(yg_precond M) {
     int32_t *done = reinterpret_cast<int32_t *>(M->d_z);
     int *d_zero = reinterpret_cast<int *>(M->d_tmp);
     YG_CUDA(cudaMemsetAsync(done, 0, sizeof(int32_t) * nb, st));
-    YG_CUDA(cudaMemsetAsync(d_zero, 0, sizeof(int), st));
+    YG_CUDA(cudaMemsetAsync(d_zero, 0, 2 * sizeof(int), st));  // (and the abort word)
     switch (B) {
     case 1: YG_TRY(ilu_factor<1>(M, done, d_zero)); break;
     case 2: YG_TRY(ilu_factor<2>(M, done, d_zero)); break;
