@@ -70,3 +70,47 @@ def test_ilu_factorizations_do_not_lower_each_others_shared_memory(ctx):
     for zs, ref in zip(together(*jobs), refs):
         for z in zs:
             assert np.array_equal(z, ref)
+
+
+def test_replayed_ilu_applies_beside_resident_solves_and_batches(ctx):
+    """ILU(0)-PCG long enough to replay its graph, resident PCG of small and of all-SM
+    systems and a resident batch, side by side: each gives what it gives alone."""
+    jobs, refs = [], []
+    c = yb.Context(0)
+    K = matrix(c, 6000, 2, 5)
+    b = yb.DeviceVector(np.random.default_rng(5).standard_normal(12000), c)
+    M = yb.ILUPreconditioner(K)
+
+    def ilu(K=K, b=b, M=M):  # (a fixed number of iterations, past the directly launched ones)
+        return [yb.solve(K, b, M=M, tol=1e-300, maxiter=100)[0].numpy() for _ in range(4)]
+    jobs.append(ilu)
+    for nb in (2000, 90000):
+        c = yb.Context(0)
+        K = matrix(c, nb, 1, 6)
+        b = yb.DeviceVector(np.random.default_rng(nb).standard_normal(nb), c)
+
+        def resident(K=K, b=b, M=yb.JacobiPreconditioner(K)):
+            return [yb.solve(K, b, M=M, tol=1e-10)[0].numpy() for _ in range(30)]
+        jobs.append(resident)
+    c = yb.Context(0)
+    B = yb.Batch(6, c)
+    slots = []
+    for i in range(6):
+        K = matrix(c, 1500 + 700 * i, 1 + i % 2, 7 + i)
+        slots.append(B.add(K, np.random.default_rng(i).standard_normal(K.rows())))
+
+    def batch():
+        out = []
+        for _ in range(8):
+            for s in slots:
+                B._keep[s][2].fill(0.0)
+            B.reset()
+            assert B.run() == 0
+            out.append(np.concatenate([B.solution(s).numpy() for s in slots]))
+        return out
+    jobs.append(batch)
+    refs = [job()[0] for job in jobs]
+    for xs, ref in zip(together(*jobs), refs):
+        assert np.all(np.isfinite(ref))
+        for x in xs:
+            assert np.array_equal(x, ref)

@@ -52,7 +52,6 @@
 
 namespace yg {
 int stream_grid(yg_context ctx, int64_t n);
-yg_status launch_cooperative(yg_context ctx, const void *kern, int grid, int threads, size_t smem, void **args);
 }
 
 enum BatchFlag : int32_t { BF_RUN = 0, BF_DONE = 1, BF_BREAK = 2, BF_NANF = 3, BF_MAXIT = 4, BF_INIT = 5, BF_EMPTY = 6 };

@@ -327,6 +327,7 @@ extern "C" yg_status yg_context_create(int32_t device, uint64_t hbm_budget_bytes
     ctx->smem_optin = prop.sharedMemPerBlockOptin;
     ctx->reduce_blocks = ctx->num_sms * 4;
     YG_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
+    ctx->stream_number = new_stream_number();
     yg_status s;
     if ((s = dev_alloc_t(ctx, &ctx->d_partials, 8 * kMaxReduceBlocks)) != YG_OK ||
         (s = dev_alloc_t(ctx, &ctx->d_scalars, 4)) != YG_OK) {

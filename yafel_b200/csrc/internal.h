@@ -88,6 +88,8 @@ struct yg_context_t {
     int32_t *d_err = nullptr;       // error word in pinned host memory (bounded waits that expired)
     long long wait_polls = 1ll << 24;  // polls of one wait of an ILU(0) kernel (seconds; a wait takes microseconds);
                                        // YAFEL_B200_WAIT_POLLS when the context is created: tests let waits expire
+    uint64_t stream_number = 0;     // of `stream`, for the turns of cooperative launches; never used again
+    int captured_blocks = 0;        // largest cooperative kernel of the capture in progress
     void *d_slots = nullptr;        // grid-wide sums of the cooperative kernels (2 x 32 bytes per block, 256
                                     // blocks), or the sums, systems and queues of a batch's (batch_resident_bytes)
     int reduce_blocks = 592;        // persistent grid for fused Krylov kernels
@@ -197,8 +199,13 @@ void flush_alloc_cache(yg_context ctx);
 yg_status allow_all_smem(yg_context ctx, const void *kern, int fixed = 0);
 // Smallest and largest row length of A into row_min / row_max, measured once.
 yg_status matrix_row_extent(yg_matrix A);
-// PCG iterations in one cooperative kernel (pcg_resident.cu)
+// Kernels whose blocks wait for one another, at most one block per SM, and graphs that
+// hold such kernels of up to `blocks` blocks (0: none): whatever context they come from,
+// their launches on a device share the SMs by count (cooperative.cu).
 yg_status launch_cooperative(yg_context ctx, const void *kern, int grid, int threads, size_t smem, void **args);
+yg_status launch_graph(yg_context ctx, cudaGraphExec_t exec, int blocks);
+uint64_t new_stream_number();
+// PCG iterations in one cooperative kernel (pcg_resident.cu)
 yg_status pcg_resident_fits(yg_matrix A, bool f32, bool jacobi, bool *fits);
 yg_status pcg_resident_launch(yg_matrix A, bool f32, const double *dinv, const double *b, double *x, double *r,
                               double *p, double *zp, int max_its, int check, double rr_replace);

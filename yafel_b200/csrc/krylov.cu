@@ -352,6 +352,7 @@ struct IterGraph {
     cudaGraphExec_t exec = nullptr;
     cudaGraph_t graph = nullptr;
     int64_t kernels = 0;
+    int blocks = 0;  // of its largest cooperative kernel
     ~IterGraph() {
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
@@ -361,12 +362,14 @@ struct IterGraph {
 template <typename F>
 static yg_status capture(yg_context ctx, int m, F &&one_iteration, IterGraph &g) {
     int64_t before = ctx->launches;
+    ctx->captured_blocks = 0;
     YG_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     yg_status s = YG_OK;
     for (int it = 0; it < m && s == YG_OK; ++it) s = one_iteration(it & 1);
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
     g.kernels = ctx->launches - before;
+    g.blocks = ctx->captured_blocks;
     ctx->launches = before;
     if (s != YG_OK) { if (graph) cudaGraphDestroy(graph); return s; }
     if (e != cudaSuccess) return fail(YG_CUDA_ERROR, "graph capture: %s", cudaGetErrorString(e));
@@ -525,7 +528,7 @@ static yg_status pcg_core(yg_matrix A, yg_precond M, const double *b, double *x,
                 YG_CUDA(cudaGetLastError());
             } else {
                 if (!g.exec) YG_TRY(capture(ctx, check_every, one, g));
-                YG_CUDA(cudaGraphLaunch(g.exec, st));
+                YG_TRY(launch_graph(ctx, g.exec, g.blocks));
                 ctx->launches += g.kernels;
             }
             YG_TRY(read_scalars(ctx, &hs));

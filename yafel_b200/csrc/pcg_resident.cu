@@ -32,8 +32,6 @@
 // do the others.
 #include "resident.cuh"
 
-#include <mutex>
-
 namespace yg {
 
 using namespace resident;
@@ -68,28 +66,6 @@ __global__ void __launch_bounds__(512, 1) k_pcg_resident(ResidentArgs a) {
             S->flag = flag;
         }
     }
-}
-
-// Cooperative kernels of two streams must not hold part of the SMs each: their
-// launches on a device follow one another, whatever context they come from.
-yg_status launch_cooperative(yg_context ctx, const void *kern, int grid, int threads, size_t smem, void **args) {
-    static std::mutex m;
-    static cudaEvent_t last[64] = {};
-    const int d = ctx->device & 63;
-    cudaStreamCaptureStatus cs;
-    YG_CUDA(cudaStreamIsCapturing(ctx->stream, &cs));
-    if (cs != cudaStreamCaptureStatusNone) {  // (an ILU(0) apply in a captured iteration: small blocks, which fit beside any)
-        YG_CUDA(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(threads), args, smem, ctx->stream));
-        YG_LAUNCHED(ctx);
-        return YG_OK;
-    }
-    std::lock_guard<std::mutex> hold(m);
-    if (last[d]) YG_CUDA(cudaStreamWaitEvent(ctx->stream, last[d], 0));
-    else YG_CUDA(cudaEventCreateWithFlags(&last[d], cudaEventDisableTiming));
-    YG_CUDA(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(threads), args, smem, ctx->stream));
-    YG_CUDA(cudaEventRecord(last[d], ctx->stream));
-    YG_LAUNCHED(ctx);
-    return YG_OK;
 }
 
 template <int B, typename VT>
