@@ -1248,7 +1248,7 @@ constexpr int kResJobs = 256;     // systems per launch
 // leave the gathers too few)
 template <int B, typename VT>
 __device__ __forceinline__ int resident_run(const BatchResident &j, int rank, resident::State &st, unsigned char *smem) {
-    return resident::pcg_run<B, VT, true>(j.m, rank, j.blocks, st, smem);
+    return resident::pcg_run<B, VT, true, false>(j.m, rank, j.blocks, st, smem);
 }
 
 __global__ void __launch_bounds__(kResThreads, kResCtas)
@@ -1587,6 +1587,10 @@ static int64_t resident_room(yg_context ctx) {
     return std::min(sm / kResCtas - 4096, (int)ctx->smem_optin - 4096);
 }
 
+static int batch_lanes(const BatchSys &d, int64_t nnzb, int G) {
+    return resident::row_lanes(d.block, (double)nnzb / d.nbrows, (d.nbrows + G - 1) / G, kResThreads);
+}
+
 // The CTAs a system's resident iterations take; 0 if it does not run resident: its share
 // must fit a CTA's shared memory.  Of a batch that more than fills the GPU the fewest CTAs
 // give the most (a CTA's time in the sums is time another system could use), of one that
@@ -1611,6 +1615,8 @@ static int resident_ctas(yg_context ctx, const BatchSys &d, int64_t nnzb) {
     // (a row that fills most of a CTA can ask for many more: four systems of 40,000 unknowns with a
     // row of 15,000 took 33.6 ms on 125 CTAs each, 19.0 on the shared kernels)
     if (G > kResMost) return 0;
+    // (nor has the batch's kernel the pass for rows much longer than the mean)
+    if (resident::has_long_rows(d.block, batch_lanes(d, nnzb, (int)G), d.row_max)) return 0;
     return resident::share(d.block, total, d.row_max, bc, rc, (int)G) <= room ? (int)G : 0;
 }
 
@@ -1692,8 +1698,7 @@ static yg_status launch_resident(yg_batch bt, int max_its) {
             m.stride = G;
             resident::costs(d.block, f32, m.corr != nullptr, true, &m.block_cost, &m.row_cost);
             m.total_cost = nnzb * m.block_cost + d.nbrows * m.row_cost;
-            m.lanes = resident::row_lanes(d.block, (double)nnzb / d.nbrows, (d.nbrows + G - 1) / G, kResThreads);
-            m.long_row = resident::long_row(d.block, m.lanes, d.row_max);
+            m.lanes = batch_lanes(d, nnzb, G);
             slots += 2 * G;
             jobs.push_back(j);
         }

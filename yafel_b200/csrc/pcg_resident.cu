@@ -48,13 +48,13 @@ struct ResidentArgs {
     const double *val64, *b;  // what a residual is replaced from
 };
 
-template <int B, typename VT>
+template <int B, typename VT, bool LONG>
 __global__ void __launch_bounds__(512, 1) k_pcg_resident(ResidentArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     KrylovScalars *S = a.S;
     if (read_flag(&S->flag)) return;  // set before the launch: the same for every block
     State st{S->tol, S->bb, S->rz0, S->maxiter, S->criterion, a.max_its, a.check, a.rr_replace, a.val64, a.b, 0, S->iter, S->rz[0], S->rr, false};
-    const int flag = pcg_run<B, VT, false>(a.sys, blockIdx.x, gridDim.x, st, smem);
+    const int flag = pcg_run<B, VT, false, LONG>(a.sys, blockIdx.x, gridDim.x, st, smem);
     if (threadIdx.x == 0) {
         if (st.timed_out) atomicExch(a.err, (int32_t)YG_TIMEOUT);
         if (blockIdx.x == 0) {
@@ -69,11 +69,14 @@ __global__ void __launch_bounds__(512, 1) k_pcg_resident(ResidentArgs a) {
 }
 
 template <int B, typename VT>
-static const void *resident_kernel() { return reinterpret_cast<const void *>(&k_pcg_resident<B, VT>); }
-static const void *resident_kernel(int B, bool f32) {
-    if (B == 1) return f32 ? resident_kernel<1, float>() : resident_kernel<1, double>();
-    if (B == 2) return f32 ? resident_kernel<2, float>() : resident_kernel<2, double>();
-    return f32 ? resident_kernel<3, float>() : resident_kernel<3, double>();
+static const void *resident_kernel(bool long_rows) {
+    return long_rows ? reinterpret_cast<const void *>(&k_pcg_resident<B, VT, true>)
+                     : reinterpret_cast<const void *>(&k_pcg_resident<B, VT, false>);
+}
+static const void *resident_kernel(int B, bool f32, bool long_rows) {
+    if (B == 1) return f32 ? resident_kernel<1, float>(long_rows) : resident_kernel<1, double>(long_rows);
+    if (B == 2) return f32 ? resident_kernel<2, float>(long_rows) : resident_kernel<2, double>(long_rows);
+    return f32 ? resident_kernel<3, float>(long_rows) : resident_kernel<3, double>(long_rows);
 }
 
 static void resident_costs(yg_matrix A, bool f32, bool jacobi, int64_t *block, int64_t *row) {
@@ -151,9 +154,9 @@ yg_status pcg_resident_launch(yg_matrix A, bool f32, const double *dinv, const d
     const int64_t rows = (A->nbrows + G - 1) / G;
     const int threads = rows * (mean > 8 ? 8 : 4) > 512 ? 512 : 256;
     m.lanes = row_lanes(A->block, mean, rows, threads);
-    m.long_row = long_row(A->block, m.lanes, A->row_max);
+    m.long_row = long_row(A->block, m.lanes);
     const size_t smem = (size_t)resident_smem(A, f32, dinv != nullptr, G);
-    const void *kern = resident_kernel(A->block, f32);
+    const void *kern = resident_kernel(A->block, f32, has_long_rows(A->block, m.lanes, A->row_max));
     YG_TRY(allow_all_smem(ctx, kern, kStaticSmem));
     YG_CUDA(cudaMemsetAsync(ctx->d_slots, 0, sizeof(SumSlot) * 2 * kMaxSumBlocks, ctx->stream));
     void *args[] = {&a};

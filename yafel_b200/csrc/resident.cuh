@@ -7,7 +7,6 @@
 #include "device_common.cuh"
 
 #include <algorithm>
-#include <climits>
 #include <cmath>
 
 namespace yg {
@@ -32,7 +31,9 @@ constexpr int gathers(int B) { return B == 1 ? 8 : (B == 2 ? 4 : 2); }
 // 2 lanes that suit a mean of 7 entries, a row of 1,000 took 62 rounds while all others
 // waited (us an iteration, streaming kernels / lanes by the mean / a warp for a long row:
 // 5,000 unknowns with a row of 1,000 21 / 32 / 12, with one of 4,000 34 / 108 / 19; 40,000 with one of
-// 15,000 84 / 406 / 67).
+// 15,000 84 / 406 / 67).  Kernels of their own (LONG) do so: with the second pass, and the
+// lanes that change between them, in the loop of all systems a solve of 4,225 unknowns
+// without long rows took 1.62 ms instead of 1.54, a batch of 24 systems 43.1 instead of 40.4.
 constexpr int kLongRounds = 4;
 // Long rows of a CTA at most: a row longer than kLongRounds * lanes * gathers(B) blocks fills 512
 // bytes of its shared memory or more.
@@ -50,7 +51,7 @@ struct System {
     int stride;
     int64_t block_cost, row_cost, total_cost;  // shared memory bytes per block, per block row, of all
     int lanes;               // lanes per block row
-    int long_row;            // rows of more blocks are long (INT_MAX: none is)
+    int long_row;            // LONG: rows of more blocks are long
 };
 struct State {
     double tol, bb, rz0;
@@ -172,12 +173,12 @@ __device__ inline int first_row(const int32_t *rowptr, int n, int64_t block_cost
 // Iterations of one system by CTA `rank` of the group's G (the same state in all of
 // them; S is one for all threads or one for each, read before the first sum and written
 // after the last); x, r and, when the flag returned is FLAG_RUN, p are written back.
-template <int B, typename VT, bool SPLIT>
+template <int B, typename VT, bool SPLIT, bool LONG>
 __device__ __forceinline__ int pcg_run(const System &a, int rank, int G, State &S, unsigned char *smem) {
     constexpr int B2 = B * B;
     __shared__ int bounds[2], nlong;
     const int tid = threadIdx.x, nt = blockDim.x;
-    if (tid == 0) nlong = 0;
+    if (LONG && tid == 0) nlong = 0;
     if (tid < 64) {
         const int64_t t = rank + (tid >> 5);
         const int r = t == G ? a.nbrows : first_row(a.rowptr, a.nbrows, a.block_cost, a.row_cost, t * a.total_cost / G);
@@ -223,7 +224,7 @@ __device__ __forceinline__ int pcg_run(const System &a, int rank, int G, State &
         q[i] = v;
         publish(i, v, 0.0);
     }
-    if (a.long_row != INT_MAX) {
+    if (LONG) {
         __syncthreads();
         if (tid < 32) {
             int n = 0;
@@ -245,19 +246,23 @@ __device__ __forceinline__ int pcg_run(const System &a, int rank, int G, State &
     double t0, t1;
     bool ok = group_sum<false, true>(a.slots + a.stride, rank, G, epoch, 0, 0, t0, t1);
     // products: `lanes` lanes a row, then a warp for each long row
-    const int passes = a.long_row != INT_MAX ? 2 : 1;
+    constexpr int passes = LONG ? 2 : 1;
+    const int L0 = a.lanes, group0 = tid / L0, ngroups0 = nt / L0;
     for (int it = 0; ok; ++it) {
         for (int i = tid; i < nd; i += nt) p[i] = fma(beta, p[i], q[i]);
         __syncthreads();  // p is read and q overwritten by other threads
         double pq = 0;
+#pragma unroll 1
         for (int pass = 0; pass < passes; ++pass) {
-            const int L = pass ? 32 : a.lanes, lane = tid & (L - 1), count = pass ? nlong : nr;
-            for (int rb = 0; rb < count; rb += nt / L) {  // the lanes of a warp take the same steps
-                int row = rb + tid / L;
+            const bool second = LONG && pass;
+            const int L = second ? 32 : L0, lane = tid & (L - 1), count = second ? nlong : nr;
+            const int group = second ? tid >> 5 : group0, ngroups = second ? nt >> 5 : ngroups0;
+            for (int rb = 0; rb < count; rb += ngroups) {  // the lanes of a warp take the same steps
+                int row = rb + group;
                 bool on = row < count;
-                if (pass && on) row = longs[row];
+                if (second && on) row = longs[row];
                 const int js = on ? rp[row] : 0, je = on ? rp[row + 1] : 0;
-                if (!pass) on = on && je - js <= a.long_row;
+                if (LONG && !second) on = on && je - js <= a.long_row;
                 double acc[B];
 #pragma unroll
                 for (int i = 0; i < B; ++i) acc[i] = 0;
@@ -349,14 +354,17 @@ __device__ __forceinline__ int pcg_run(const System &a, int rank, int G, State &
             ++epoch;
             if (!(ok = group_sum<false, true>(a.slots, rank, G, epoch, 0, 0, t0, t1))) break;
             srz = srr = 0;
+#pragma unroll 1
             for (int pass = 0; pass < passes; ++pass) {
-                const int L = pass ? 32 : a.lanes, lane = tid & (L - 1), count = pass ? nlong : nr;
-                for (int rb = 0; rb < count; rb += nt / L) {
-                    int row = rb + tid / L;
+                const bool second = LONG && pass;
+                const int L = second ? 32 : L0, lane = tid & (L - 1), count = second ? nlong : nr;
+                const int group = second ? tid >> 5 : group0, ngroups = second ? nt >> 5 : ngroups0;
+                for (int rb = 0; rb < count; rb += ngroups) {
+                    int row = rb + group;
                     bool on = row < count;
-                    if (pass && on) row = longs[row];
+                    if (second && on) row = longs[row];
                     const int js = on ? rp[row] : 0, je = on ? rp[row + 1] : 0;
-                    if (!pass) on = on && je - js <= a.long_row;
+                    if (LONG && !second) on = on && je - js <= a.long_row;
                     double acc[B];
 #pragma unroll
                     for (int i = 0; i < B; ++i) acc[i] = 0;
@@ -421,11 +429,9 @@ inline int64_t share(int B, int64_t total_cost, int64_t row_max, int64_t block_c
     return (total_cost + G - 1) / G + row_max * block_cost + row_cost + 256 + list;
 }
 
-// The row length above which a row takes a warp.
-inline int long_row(int B, int lanes, int64_t row_max) {
-    const int n = kLongRounds * lanes * gathers(B);
-    return lanes < 32 && row_max > n ? n : INT_MAX;
-}
+// The row length above which a row takes a warp, and whether a system has such rows.
+inline int long_row(int B, int lanes) { return kLongRounds * lanes * gathers(B); }
+inline bool has_long_rows(int B, int lanes, int64_t row_max) { return lanes < 32 && row_max > long_row(B, lanes); }
 
 // Lanes per block row: one round of gathers each, more where the threads allow.
 inline int row_lanes(int B, double mean, int64_t rows, int threads) {
