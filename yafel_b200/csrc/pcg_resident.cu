@@ -95,7 +95,12 @@ static int64_t resident_smem(yg_matrix A, bool f32, bool jacobi, int G) {
 // 8.9 on 148: every block polls every other's words) and the products 0.52 ns per CSR
 // entry, 0.27 ns per entry of a block, divided by the blocks (40,401 unknowns, 361,201
 // entries: 10.7 us on 32, 8.3 on 64, 8.4 on 96, 10.0 on 148), so the best number grows
-// with the square root of the entries; the shared memory sets a lower bound.
+// with the square root of the entries; the shared memory sets a lower bound.  Solves of
+// several contexts run side by side as far as their blocks fit the SMs (solves a second
+// with 1, 2, 4, 8 threads, streaming iterations -> these: 4,225 unknowns 201, 322, 458, 490 ->
+// 527, 1007, 2000, 2359; 30,258 of order-2 plane elasticity 32, 49, 62, 58 -> 53 whatever the
+// threads; 150,000 of order-2 Poisson 15, 22, 27, 26 -> 22).  Half the SMs for the second
+// would let two run at once, 102 a second, but a solve alone takes 1.9 % longer.
 static int resident_blocks(yg_matrix A, bool f32, bool jacobi) {
     yg_context ctx = A->ctx;
     const double entries = (double)A->nnzb * A->block * A->block;

@@ -391,7 +391,8 @@ static yg_status ilu_factor(yg_precond M, int32_t *done, int *zeros) {
     YG_TRY(allow_all_smem(ctx, reinterpret_cast<const void *>(kern)));
     Waits waits = waits_of(M);
     void *args[] = {&nb, &M->d_lower_rows, &A->d_rowptr, &A->d_col, &A->d_diag, &M->d_lu, &done, &zeros, &room, &waits};
-    return launch_cooperative(ctx, reinterpret_cast<const void *>(kern), ctx->num_sms, 32 * warps, (size_t)smem, args);
+    return launch_cooperative(ctx, reinterpret_cast<const void *>(kern), std::min(ctx->num_sms, (nb + warps - 1) / warps), 32 * warps,
+                              (size_t)smem, args);
 }
 
 // (flag: set when the solver that captured the apply has stopped)
@@ -418,7 +419,8 @@ static yg_status ilu_apply(yg_precond M, const double *r, double *z, const int32
     case 7: kern = reinterpret_cast<const void *>(&k_ilu_apply<7>); break;
     default: kern = reinterpret_cast<const void *>(&k_ilu_apply<8>); break;
     }
-    YG_TRY(launch_cooperative(ctx, kern, ctx->num_sms, kThreads, 0, args));
+    const int grid = (int)std::min<int64_t>(ctx->num_sms, (nb + kThreads / 32 - 1) / (kThreads / 32));
+    YG_TRY(launch_cooperative(ctx, kern, grid, kThreads, 0, args));
     YG_CUDA(cudaGetLastError());
     return YG_OK;
 }
