@@ -64,6 +64,10 @@ struct yg_dofmap_t {
     int32_t *d_ncol = nullptr;
     int64_t nnz_nodes = 0;
     std::vector<ElementGroup> groups;
+    // scatter maps that were given up for memory are laid out again at an assembly, the
+    // first time after 4 assemblies without, then 8, 16, ... (laying out costs a few)
+    bool mappable = false;
+    int unmapped = 0, map_wait = 4;
 };
 
 namespace yg {
@@ -938,11 +942,11 @@ static yg_status build_pattern(yg_dofmap d, int nsd) {
     for (size_t g = 0; mapped && g < d->groups.size(); ++g) {
         ElementGroup &gr = d->groups[g];
         const size_t cells = gr.color_ptr.empty() ? 0 : (size_t)gr.color_ptr.back();
-        mapped = dev_alloc_t(ctx, &gr.d_map, cells * gr.tab.nen * gr.tab.nen) == YG_OK;
+        mapped = dev_alloc_optional(ctx, &gr.d_map, cells * gr.tab.nen * gr.tab.nen) == YG_OK;
         maps.map[g] = gr.d_map;
         maps.nen[g] = gr.tab.nen;
     }
-    mapped = mapped && dev_alloc_t(ctx, &d_slot, nc + 1) == YG_OK && dev_alloc_t(ctx, &d_rank, nc + 1) == YG_OK;
+    mapped = mapped && dev_alloc_optional(ctx, &d_slot, nc + 1) == YG_OK && dev_alloc_optional(ctx, &d_rank, nc + 1) == YG_OK;
     if (mapped) {
         for (size_t g = 0; g < d->groups.size(); ++g) {
             const ElementGroup &gr = d->groups[g];
@@ -968,15 +972,72 @@ static yg_status build_pattern(yg_dofmap d, int nsd) {
 #undef TRYC
     if (e != cudaSuccess) return fail(YG_CUDA_ERROR, "pattern build: %s", cudaGetErrorString(e));
     for (auto &g : d->groups) {
-        if (mapped && !odd) {
-            ctx->optional.push_back(reinterpret_cast<void **>(&g.d_map));
-        } else {
+        if (!mapped || odd) {
+            dev_free(ctx, g.d_map);
+            g.d_map = nullptr;
+        }
+        if (!odd) ctx->optional.push_back(reinterpret_cast<void **>(&g.d_map));
+    }
+    d->mappable = nn > 0 && !d->groups.empty() && !odd;
+    d->unmapped = 0;
+    d->map_wait = 4;
+    d->nnz_nodes = nnz;
+    d->pattern_nsd = nsd;
+    return YG_OK;
+}
+
+// Scatter map entries of the cells of one colour, of rank `rank`, from the pattern: the
+// first pass, of all colours, marks every entry with the lowest rank that touches it, the
+// second writes positions and first touches.
+__global__ void k_map_again(const int32_t *__restrict__ order, int ncell, int nen, const int32_t *__restrict__ off,
+                            const int32_t *__restrict__ el, const int32_t *__restrict__ nrp, const int32_t *__restrict__ ncol,
+                            unsigned *__restrict__ low, unsigned rank, uint16_t *__restrict__ map, int pass) {
+    const int64_t n = (int64_t)ncell * nen * nen;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int t = (int)(i / (nen * nen)), ab = (int)(i - (int64_t)t * nen * nen), base = off[order[t]];
+        const int row = el[base + ab / nen], k = find_col(ncol, nrp[row], nrp[row + 1], el[base + ab % nen]);
+        if (pass == 0) atomicMin(low + k, rank);
+        else map[i] = (uint16_t)((k - nrp[row]) | (low[k] == rank ? 0x8000 : 0));
+    }
+}
+
+static bool has_maps(yg_dofmap d) {
+    bool all = true;
+    for (const ElementGroup &g : d->groups) all = all && g.d_map;
+    return all;
+}
+
+// Lays the scatter maps out again where memory allows (they were given up, or found none).
+static yg_status restore_maps(yg_dofmap d) {
+    yg_context ctx = d->ctx;
+    unsigned *low = nullptr;
+    auto cells = [](const ElementGroup &g) { return g.color_ptr.empty() ? 0 : (size_t)g.color_ptr.back(); };
+    bool room = dev_alloc_optional(ctx, &low, d->nnz_nodes + 1) == YG_OK;
+    for (ElementGroup &g : d->groups)
+        room = room && (g.d_map || dev_alloc_optional(ctx, &g.d_map, cells(g) * g.tab.nen * g.tab.nen) == YG_OK);
+    if (room) {
+        YG_CUDA(cudaMemsetAsync(low, 0xff, sizeof(unsigned) * (d->nnz_nodes + 1), ctx->stream));
+        for (int pass = 0; pass < 2; ++pass)
+            for (size_t g = 0; g < d->groups.size(); ++g) {
+                const ElementGroup &gr = d->groups[g];
+                const int nen = gr.tab.nen;
+                for (size_t c = 0; c + 1 < gr.color_ptr.size(); ++c) {
+                    const int first = gr.color_ptr[c], n = gr.color_ptr[c + 1] - first;
+                    if (n == 0) continue;
+                    k_map_again<<<stream_grid(ctx, (int64_t)n * nen * nen), kThreads, 0, ctx->stream>>>(
+                        gr.d_order + first, n, nen, d->d_offsets, d->d_elements, d->d_nrowptr, d->d_ncol, low,
+                        (unsigned)(64 * g + c), gr.d_map + (size_t)first * nen * nen, pass);
+                    YG_LAUNCHED(ctx);
+                }
+            }
+        YG_CUDA(cudaGetLastError());
+    } else {
+        for (ElementGroup &g : d->groups) {
             dev_free(ctx, g.d_map);
             g.d_map = nullptr;
         }
     }
-    d->nnz_nodes = nnz;
-    d->pattern_nsd = nsd;
+    dev_free(ctx, low);
     return YG_OK;
 }
 
@@ -1404,10 +1465,13 @@ extern "C" yg_status yg_assemble(yg_dofmap d, const yg_physics *physics, uint32_
             return fail(YG_BAD_ARG, "matrix was not assembled from this dofmap in this format");
         }
         yg_matrix A = *K;
+        if (d->mappable && !has_maps(d) && ++d->unmapped >= d->map_wait) {
+            YG_TRY(restore_maps(d));
+            d->unmapped = 0;
+            d->map_wait = std::min(2 * d->map_wait, 1 << 20);
+        }
         // with scatter maps every entry is stored before it is added to
-        bool mapped = true;
-        for (const ElementGroup &g : d->groups) mapped = mapped && g.d_map;
-        if (!mapped || d->groups.empty())
+        if (!has_maps(d) || d->groups.empty())
             YG_CUDA(cudaMemsetAsync(A->d_val, 0, sizeof(double) * A->nnzb * A->block * A->block, ctx->stream));
         val = A->d_val;
     }

@@ -51,21 +51,26 @@ void flush_alloc_cache(yg_context ctx) {
     ctx->cached_bytes = 0;
 }
 
-// Frees the context's optional buffers; whether there were any.
-static bool release_optional(yg_context ctx) {
-    bool any = false;
+static size_t optional_bytes(yg_context ctx) {
+    size_t n = 0;
+    for (void **p : ctx->optional)
+        if (*p) n += ctx->allocs[*p];
+    return n;
+}
+
+static void release_optional(yg_context ctx) {
     for (void **p : ctx->optional) {
-        any = any || *p;
         dev_free(ctx, *p);
         *p = nullptr;
     }
-    return any;
 }
 
-yg_status dev_alloc(yg_context ctx, void **p, size_t bytes) {
+// optional: the caller does without when there is no room, so nothing else goes for it.
+yg_status dev_alloc(yg_context ctx, void **p, size_t bytes, bool optional) {
     *p = nullptr;
     if (bytes == 0) bytes = 16;
-    if (ctx->budget && ctx->in_use + bytes > ctx->budget) release_optional(ctx);
+    const size_t extra = optional ? 0 : optional_bytes(ctx);  // what this allocation may have freed
+    if (ctx->budget && ctx->in_use + bytes > ctx->budget && ctx->in_use - extra + bytes <= ctx->budget) release_optional(ctx);
     if (ctx->budget && ctx->in_use + bytes > ctx->budget)
         return fail(YG_OVER_BUDGET, "allocation of %zu bytes exceeds the HBM budget (%llu of %llu in use)",
                     bytes, (unsigned long long)ctx->in_use, (unsigned long long)ctx->budget);
@@ -84,8 +89,10 @@ yg_status dev_alloc(yg_context ctx, void **p, size_t bytes) {
             flush_alloc_cache(ctx);
             e = cudaMalloc(p, bytes);
         }
-        if (e != cudaSuccess && release_optional(ctx)) {
+        size_t left = 0, all = 0;
+        if (e != cudaSuccess && extra && cudaMemGetInfo(&left, &all) == cudaSuccess && left + extra >= bytes) {
             cudaGetLastError();
+            release_optional(ctx);
             flush_alloc_cache(ctx);
             e = cudaMalloc(p, bytes);
         }

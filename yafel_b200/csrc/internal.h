@@ -78,8 +78,8 @@ struct yg_context_t {
     std::multimap<size_t, CachedBlock> cache;
     size_t cached_bytes = 0;
     // buffers that calls do without when memory is short (an assembly's scatter
-    // map): an allocation that would fail frees them all (the pointers become
-    // NULL) and tries again
+    // map): an allocation that their bytes would let succeed frees them all (the
+    // pointers become NULL)
     std::vector<void **> optional;
     // reduction scratch (device) and pinned host mailbox
     double *d_partials = nullptr;   // 8 * kMaxReduceBlocks doubles
@@ -159,11 +159,15 @@ struct yg_precond_t {
 namespace yg {
 
 size_t batch_resident_bytes(yg_context ctx);
-yg_status dev_alloc(yg_context ctx, void **p, size_t bytes);
+yg_status dev_alloc(yg_context ctx, void **p, size_t bytes, bool optional = false);
 void dev_free(yg_context ctx, void *p);
 template <typename T>
 yg_status dev_alloc_t(yg_context ctx, T **p, size_t count) {
     return dev_alloc(ctx, reinterpret_cast<void **>(p), count * sizeof(T) + 16);
+}
+template <typename T>
+yg_status dev_alloc_optional(yg_context ctx, T **p, size_t n) {
+    return dev_alloc(ctx, reinterpret_cast<void **>(p), n * sizeof(T) + 16, true);
 }
 
 // ---- kernels-side entry points (implemented in .cu files) ----

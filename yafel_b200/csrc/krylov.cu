@@ -593,7 +593,7 @@ yg_status solve_cg(yg_matrix A, yg_precond M, yg_vector bv, yg_vector xv, const 
     bool resident = false;
     if (precond_fusable(M) && !o.profile)
         YG_TRY(pcg_resident_fits(A, o.precision != YG_PREC_FP64, precond_dinv(M) != nullptr, &resident));
-    if (resident && alloc_vec(ctx, &w.zp, 2 * n) != YG_OK) resident = false;  // no room beside the budget
+    if (resident && dev_alloc_optional(ctx, &w.zp, 2 * n) != YG_OK) resident = false;  // no room beside the budget
     if (!resident) YG_TRY(spmv_autotune_device(A));  // the FP32-value kernel has its own tuning
     if (!resident && o.precision != YG_PREC_FP64 && (A->block == 2 || A->block == 3)) {
         // FP32 gather copy of p (node-padded) for the FP32-value TMA SpMV
