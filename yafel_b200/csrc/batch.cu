@@ -44,6 +44,7 @@
 #include "internal.h"
 #include "device_common.cuh"
 #include "resident.cuh"
+#include "resident_queues.h"
 
 #include <algorithm>
 #include <cmath>
@@ -1241,7 +1242,12 @@ constexpr int kResThreads = 256;  // 254 registers, no spills (384: 59.1 ms, 512
 // 14 of up to 20,000: 42, 13, 13, 13).
 constexpr int kResMost = 48;
 constexpr int kResCheck = 16;     // iterations between looks at a due replacement
-constexpr int kResQueue = 8;      // systems per CTA and launch: bounds what a CTA waits for another
+// Systems one after the other per CTA and launch, and longest chain of systems that wait for
+// one another's CTAs: a CTA waits for its group at most 7 systems of kResRun iterations
+// of up to 100 us (a row of 15,000 entries; 10 us are usual), 2.9 s.  A sum's poll
+// limit is 2^22, above 4 s: after 4,096 polls each sleeps a microsecond.
+constexpr int kResQueue = 8;
+constexpr int kResRun = 1 << 12;  // iterations of a system per launch
 constexpr int kResJobs = 256;     // systems per launch
 
 // (the system's description and state stay in shared memory: in registers they would
@@ -1649,35 +1655,15 @@ static yg_status launch_resident(yg_batch bt, int max_its) {
         if (sys_live(bt, s) && bt->sys[s].resident) todo.push_back(s);
     std::stable_sort(todo.begin(), todo.end(), [&](int a, int b) { return cost(a) > cost(b); });
     while (!todo.empty()) {
-        // the longest system that the free CTAs can take starts first; when there is none,
-        // on to the next time at which CTAs become free
+        std::vector<ResidentJob> want;
+        for (int s : todo) want.push_back({bt->sys[s].resident, cost(s)});
+        const ResidentQueues plan = place_resident(want, ctas, kResQueue, kResJobs);
         std::vector<BatchResident> jobs;
-        std::vector<std::vector<int2>> queue(ctas);
-        std::vector<double> until(ctas, 0.0);
-        double now = 0;
         int64_t slots = 0;
-        for (;;) {
-            std::vector<int> free;
-            for (int c = 0; c < ctas; ++c)
-                if (until[c] <= now && queue[c].size() < (size_t)kResQueue) free.push_back(c);
-            size_t k = 0;
-            while (k < todo.size() && bt->sys[todo[k]].resident > (int)free.size()) ++k;
-            if (k == todo.size() || jobs.size() == (size_t)kResJobs) {
-                double next = 1e300;
-                for (int c = 0; c < ctas; ++c)
-                    if (until[c] > now && queue[c].size() < (size_t)kResQueue) next = std::min(next, until[c]);
-                if (todo.empty() || next == 1e300 || jobs.size() == (size_t)kResJobs) break;
-                now = next;
-                continue;
-            }
-            const int s = todo[k];
-            todo.erase(todo.begin() + k);
+        for (int at : plan.placed) {
+            const int s = todo[at];
             const BatchSys &d = bt->sys[s];
             const int G = d.resident;
-            for (int i = 0; i < G; ++i) {
-                until[free[i]] = now + cost(s);
-                queue[free[i]].push_back(make_int2((int)jobs.size(), i));
-            }
             const bool f32 = d.precision == YG_PREC_MIXED;
             const int64_t nnzb = bt->nnzb[s];
             BatchResident j{};
@@ -1705,7 +1691,7 @@ static yg_status launch_resident(yg_batch bt, int max_its) {
         std::vector<int32_t> begin(1, 0);
         std::vector<int2> entries;
         for (int c = 0; c < ctas; ++c) {
-            entries.insert(entries.end(), queue[c].begin(), queue[c].end());
+            for (const auto &e : plan.queue[c]) entries.push_back(make_int2(e.first, e.second));
             begin.push_back((int32_t)entries.size());
         }
         YG_CUDA(cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(BatchResident) * jobs.size(), cudaMemcpyHostToDevice, ctx->stream));
@@ -1723,6 +1709,10 @@ static yg_status launch_resident(yg_batch bt, int max_its) {
         const int room = (int)resident_room(ctx);
         YG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
         YG_TRY(launch_cooperative(ctx, kern, ctas, kResThreads, (size_t)room, args));
+        std::vector<int> rest;
+        for (size_t i = 0; i < todo.size(); ++i)
+            if (std::find(plan.placed.begin(), plan.placed.end(), (int)i) == plan.placed.end()) rest.push_back(todo[i]);
+        todo.swap(rest);
     }
     return YG_OK;
 }
@@ -2070,7 +2060,7 @@ extern "C" yg_status yg_batch_run(yg_batch bt, int32_t max_blocks, int32_t *n_ac
     YG_TRY(batch_prepare(bt));
     int active = 0;
     for (int blk = 0; max_blocks <= 0 || blk < max_blocks; ++blk) {
-        YG_TRY(batch_launch(bt, max_blocks <= 0 ? 1 << 12 : bt->m));  // (0: nobody looks at the systems in between)
+        YG_TRY(batch_launch(bt, max_blocks <= 0 ? kResRun : bt->m));  // (0: nobody looks at the systems in between)
         YG_TRY(batch_collect(bt, &active));
         if (active == 0) break;
     }
