@@ -606,7 +606,7 @@ k_assemble(const int32_t *__restrict__ order, int ncell, const uint16_t *__restr
                 ta = tl / nt;
                 tb = tl - ta * nt;
             }
-            const bool both = SYM && ta != tb;
+            const bool both = SYM && ta != tb, diag = SYM && ta == tb;
             // where node pair (A, B), A the row, lies: its position with bit 31 clear
             // when it is stored, set when it is added to; -1 when there is none
             auto position = [&](int A, int B) -> int {
@@ -633,7 +633,10 @@ k_assemble(const int32_t *__restrict__ order, int ncell, const uint16_t *__restr
                     const int hi = 4 * h + (lane >> 3), lo = lane & 7;
                     const int a = E == 1 ? (f ? rb + h : ra) : (f || !by_col ? hi : lo);
                     const int b = E == 1 ? (f ? ra : rb + h) : (f || !by_col ? lo : hi);
-                    pos[2 * f + h] = f && !both ? -1 : position(8 * (f ? tb : ta) + a, 8 * (f ? ta : tb) + b);
+                    // (E == 1: a diagonal tile stores its pairs with ra <= rb + h, and those below the
+                    // diagonal as their transposes, so that the tangent is symmetric to the bit)
+                    const bool off = E == 1 ? (f ? !SYM || (diag && ra >= rb + h) : diag && ra > rb + h) : f && !both;
+                    pos[2 * f + h] = off ? -1 : position(8 * (f ? tb : ta) + a, 8 * (f ? ta : tb) + b);
                 }
             double C[NC][2];
 #pragma unroll
@@ -729,11 +732,24 @@ k_assemble(const int32_t *__restrict__ order, int ncell, const uint16_t *__restr
                     for (int h = 0; h < 2; ++h) {
                         const int pair = f || by_col ? (rb + h) * 8 + ra : ra * 8 + rb + h;
                         double *o = tile + pair * E + (pair >> 4);
+                        // a diagonal tile's pairs below the diagonal are the transposes of those above,
+                        // and so are the entries of the pairs on it
+                        const int side = diag ? ra - (rb + h) : -1;
+                        if (side <= 0) {
 #pragma unroll
-                        for (int i = 0; i < DPN; ++i)
+                            for (int i = 0; i < DPN; ++i)
 #pragma unroll
-                            for (int k = 0; k < DPN; ++k)
-                                o[i * DPN + k] = f ? C[(k * DPN + i) % NC][h] : C[(i * DPN + k) % NC][h];
+                                for (int k = 0; k < DPN; ++k)
+                                    o[i * DPN + k] = f || (side == 0 && i > k) ? C[(k * DPN + i) % NC][h] : C[(i * DPN + k) % NC][h];
+                        }
+                        if (diag && side < 0) {
+                            const int mirror = (rb + h) * 8 + ra;
+                            double *t = tile + mirror * E + (mirror >> 4);
+#pragma unroll
+                            for (int i = 0; i < DPN; ++i)
+#pragma unroll
+                                for (int k = 0; k < DPN; ++k) t[i * DPN + k] = C[(k * DPN + i) % NC][h];
+                        }
                     }
                     __syncwarp();
 #pragma unroll
