@@ -191,8 +191,9 @@ enum { SP_CG = 0, SP_VERIFY = 1, SP_BICG_V = 2, SP_BICG_T = 3 };
 enum { ACT_ITER = 0, ACT_VERIFY = 1, ACT_RESTART = 2, ACT_RESIDENT = 3 };
 __device__ __forceinline__ int activity(const BatchScal *sc, int kind) {
     const volatile BatchScal *v = sc;
-    const int flag = v->flag, stop = v->stop, rep = v->replace, rst = v->restart;
-    if (kind == ACT_ITER) return flag == BF_RUN && stop == BS_NONE && !v->resident;
+    // (all loads at once: one that waits for another's value costs every item a trip to L2)
+    const int flag = v->flag, stop = v->stop, rep = v->replace, rst = v->restart, resident = v->resident;
+    if (kind == ACT_ITER) return flag == BF_RUN && stop == BS_NONE && !resident;
     if (kind == ACT_RESIDENT) return flag == BF_RUN && stop == BS_NONE;
     if (kind == ACT_VERIFY) return (flag == BF_INIT) || (flag == BF_RUN && (stop == BS_CONV || rep));
     return rst != 0;
