@@ -392,7 +392,8 @@ YG_API yg_status yg_bicgstab(yg_matrix A, yg_precond M, yg_vector b, yg_vector x
  * yg_batch_add waits for that context's pending work, and the caller frees them
  * only after the slot is removed between a wait and the next launch.  Systems may be added and removed between calls of
  * yg_batch_run (continuous batching); work advances in blocks of iterations
- * captured in one CUDA graph followed by an FP64 verification pass (true
+ * (16, captured in one CUDA graph; 128 of the PCG systems that iterate in the SMs'
+ * shared memory) followed by an FP64 verification pass (true
  * residual b - A x for converged systems, BiCGSTAB restarts after a breakdown,
  * and the residual replacement of YG_PREC_MIXED).  A system's result does not
  * depend on the other systems in the batch. */

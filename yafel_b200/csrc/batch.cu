@@ -1219,28 +1219,31 @@ __global__ void k_batch_jacobi(int64_t nbrows, int B, const int32_t *__restrict_
 // An iteration of the kernels above is four launches (PCG, two block sizes) whatever the systems' sizes, each
 // of which waits for the slowest of them.  A PCG system whose matrix fits the shared
 // memory of some CTAs is iterated by one cooperative kernel instead: it has its own
-// group of CTAs, which hold its matrix and vectors and iterate for a block (m
-// iterations; to its end when nobody looks at the systems in between) or until it
+// group of CTAs, which hold its matrix and vectors and iterate for a block
+// (kResBlocks of m iterations; to its end when nobody looks at the systems in between) or until it
 // stops; a mixed-precision residual is replaced on the way.  The verification pass then decides as
 // after a block.  A CTA takes the systems of its queue in the order in which the host
 // placed them, the same order in all queues, so the first system that is not done
 // always has all its CTAs.  A group's size follows from the system alone and a block's
 // end changes no bit of its iterates, so its result does not depend on the others.
-// Measured, before -> now: 14 systems of up to 20,000 unknowns of 2D problems 44 -> 13 ms;
-// 8 of up to 10,000: 21.6 -> 6.5; 3 of up to 4,000: 7.7 -> 2.9.  The trips through L2 of
+// Measured, shared kernels -> resident: 14 systems of up to 20,000 unknowns of 2D problems 52 -> 17.5
+// ms; 8 of up to 10,000: 37.7 -> 10.5; 3 of up to 4,000: 20.5 -> 5.5.  The trips through L2 of
 // the sums and the gathers bound it.
 struct BatchResident {
     resident::System m;
     int32_t sys, blocks;  // slot; CTAs of the group
 };
 
-constexpr int kResCtas = 1;       // CTAs per SM (two of 128 threads: 51.0 ms where one of 256 takes 47.9)
-constexpr int kResThreads = 256;  // 254 registers, no spills (384: 59.1 ms, 512: 92)
+// 24 systems of up to 40,000 unknowns take 40.4 ms, 64 of up to 100,000 437 ms (as do the figures
+// below, unless they say otherwise).  Two CTAs of 128 threads: 97.7 and 419, fewer of the
+// larger ones fit; 384 threads: 38.8 and 440; 512: 66.1 and 506.
+constexpr int kResCtas = 1;       // CTAs per SM
+constexpr int kResThreads = 256;  // 255 registers, no spills
 // Systems whose FP64 matrix and vectors fill at most this many CTAs run resident.  Many
 // larger ones keep the shared kernels busy, which then take less of the GPU's time for
-// each: 128 systems of 1,000 to 200,000 unknowns take 1.29 s without the resident kernel,
-// 1.29 with 48, 1.46 with 80 and 1.75 with 148 (24 of up to 40,000: 97 ms, 91, 49, 49;
-// 14 of up to 20,000: 42, 13, 13, 13).
+// each (ms with none resident / 24 / 48 / 80: 14 of up to 20,000 unknowns 52 / 58 / 18 / 18; 24 of up
+// to 40,000 88 / 91 / 40 / 40, of another draw 95 / 99 / 87 / 48; 64 of up to 100,000 423 / 421 / 431 /
+// 538; 128 of up to 200,000 1599 / 1609 / 1611 / 1666; 40 of up to 400,000 1724 / 1726 / 1724 / 1755).
 constexpr int kResMost = 48;
 constexpr int kResCheck = 16;     // iterations between looks at a due replacement
 // Systems one after the other per CTA and launch, and longest chain of systems that wait for
@@ -1249,6 +1252,14 @@ constexpr int kResCheck = 16;     // iterations between looks at a due replaceme
 // limit is 2^22, above 4 s: after 4,096 polls each sleeps a microsecond.
 constexpr int kResQueue = 8;
 constexpr int kResRun = 1 << 12;  // iterations of a system per launch
+// Blocks of m iterations that a resident system does in one block of the others when a
+// program steps through a batch.  A launch loads every matrix into shared memory again and
+// waits for its longest queue (ms of stepped solves, no resident kernel / 1 block / 2 / 4 / 8: 3
+// systems of up to 4,000 unknowns 22 / 9.2 / 7.3 / 6.5 / 5.9; 24 of up to 40,000 91 / 60 / 52 / 49 / 47;
+// 64 of up to 100,000 433 / 474 / 451 / 440 / 433; 128 of up to 200,000 1615 / 1675 / 1646 / 1633 / 1626;
+// 40 of up to 400,000 1735 / 1766 / 1762 / 1757 / 1755).  More than 8, about a millisecond, would
+// hold up the systems that finish and what the program does between blocks.
+constexpr int kResBlocks = 8;
 constexpr int kResJobs = 256;     // systems per launch
 
 // (the system's description and state stay in shared memory: in registers they would
@@ -1602,9 +1613,9 @@ static int batch_lanes(const BatchSys &d, int64_t nnzb, int G) {
 // must fit a CTA's shared memory.  Of a batch that more than fills the GPU the fewest CTAs
 // give the most (a CTA's time in the sums is time another system could use), of one that
 // does not, about the number a system alone would take (pcg_resident.cu).  0.4 of that
-// number lies between: 24 systems of 1,000 to 40,000 unknowns, all resident, take 47.9 ms
-// with 0.3 of it, 51.1 with 0.4, 60.4 with 0.5 and 62.7 with 0.6; 8 of up to 10,000 take 7.4, 6.7, 6.2 and
-// 5.9; 3 of up to 40,000 take 15.1, 13.8, 12.1 and 11.0.
+// number lies between (ms with 0.3 / 0.4 / 0.5 / 0.6 / 1: 24 systems of up to 40,000 unknowns 40.2 / 40.4 /
+// 76 / 100 / 108, the larger ones then passing kResMost; 8 of up to 10,000 11.2 / 10.5 / 9.3 / 8.4 / 39; 3
+// of up to 4,000 6.4 / 5.5 / 5.5 / 5.2 / 5.2).
 static int resident_ctas(yg_context ctx, const BatchSys &d, int64_t nnzb) {
     if (d.method != BM_CG || d.solo || d.nbrows < 1 || d.nbrows >= (1 << 24)) return 0;
     const int64_t room = resident_room(ctx);
@@ -2061,7 +2072,7 @@ extern "C" yg_status yg_batch_run(yg_batch bt, int32_t max_blocks, int32_t *n_ac
     YG_TRY(batch_prepare(bt));
     int active = 0;
     for (int blk = 0; max_blocks <= 0 || blk < max_blocks; ++blk) {
-        YG_TRY(batch_launch(bt, max_blocks <= 0 ? kResRun : bt->m));  // (0: nobody looks at the systems in between)
+        YG_TRY(batch_launch(bt, max_blocks <= 0 ? kResRun : kResBlocks * bt->m));  // (0: nobody looks at the systems in between)
         YG_TRY(batch_collect(bt, &active));
         if (active == 0) break;
     }
@@ -2072,7 +2083,7 @@ extern "C" yg_status yg_batch_run(yg_batch bt, int32_t max_blocks, int32_t *n_ac
 extern "C" yg_status yg_batch_launch(yg_batch bt) {
     if (!bt) return fail(YG_BAD_ARG, "yg_batch_launch: NULL batch");
     YG_TRY(batch_prepare(bt));
-    return batch_launch(bt, bt->m);
+    return batch_launch(bt, kResBlocks * bt->m);
 }
 
 extern "C" yg_status yg_batch_wait(yg_batch bt, int32_t *n_active) {

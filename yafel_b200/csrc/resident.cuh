@@ -23,8 +23,8 @@ struct alignas(32) SumSlot {
 // Blocks of a row that a lane gathers at a time: a round costs a trip to L2 whatever
 // their number, and there are rows x lanes / threads rounds.  Against 4, 2 and 2 (us an
 // iteration): 40,401 unknowns of Q1 8.2 -> 7.6, of Q2 8.9 -> 9.5, 44,521 of Q3 11.7 -> 11.3,
-// 45,602 of order-3 plane elasticity 13.3 -> 12.6; a batch of 24 systems gains most (59.4 ms with 6, 3
-// and 2, 51.1 with these).
+// 45,602 of order-3 plane elasticity 13.3 -> 12.6; batches of 24 systems 47.7 -> 40.4 and 93.5 -> 88.6 ms (39.8
+// and 94.0 with 6, 3 and 2).
 constexpr int gathers(int B) { return B == 1 ? 8 : (B == 2 ? 4 : 2); }
 
 // A row of more than kLongRounds rounds of its lanes is left to a whole warp: with the
