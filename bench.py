@@ -1030,12 +1030,26 @@ def cpu_problems(specs, meshes=None, budget_s=30.0, max_dofs=None):
                       % (n, dofs, t, max(rels))}
 
 
+def reference_library():
+    """Whether the reference's code compiled in place (oracle/_ref) is here, built now if
+    its sources are."""
+    from oracle import oracle as O
+    if not O.ref_available():
+        try:
+            O.build()
+        except Exception:
+            return False
+    return O.ref_available()
+
+
 def cpu_baseline(args):
     """One calibrated sample of the reference's CPU path (untimed probe solve
     first) on the whole cpu_nx^3 cube, scaled to the configured size the way
     the reference arm scales its sample (phases up to the solve by the element
     count, the solve by stored entries times iterations), reported beside the
-    GPU numbers."""
+    GPU numbers (None without the reference's library)."""
+    if not reference_library():
+        return None
     threads = os.cpu_count() or 1
     nx = args.cpu_nx
     tol, _ = calibrate_cpu_tol(nx, threads)
@@ -1068,6 +1082,10 @@ def run_reference(args):
     W-1 runs at 16^3."""
     ws, rank, _ = dist_env()
     if rank != 0:
+        return
+    if not reference_library():
+        print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref/libyafel_ref.so is absent and the "
+                          "reference's sources to build it from are not here"}), flush=True)
         return
     threads = os.cpu_count() or 1
     rnx = args.ref_nx
