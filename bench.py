@@ -459,20 +459,22 @@ def assembly_flops_per_element(nq, nen, dpn, nsd):
 
 
 def assembly_executed_flops_per_element(nq, nen, nsd):
-    """Flops k_assemble executes per 3D elasticity element: per quadrature point
-    the Jacobian (nen*nsd^2 multiply-adds) and its inverse (~60), the physical
-    gradients (nen*nsd^2 multiply-adds), and per node pair of the upper triangle
-    (nen(nen+1)/2) and point the dot product (6) and the scaled weight (1) plus
-    8 flops for each of the nsd^2 block entries."""
-    geometry = nq * (2 * nen * nsd * nsd + 60) + nq * nen * 2 * nsd * nsd
-    pairs = nen * (nen + 1) // 2
-    return geometry + pairs * nq * (7 + 8 * nsd * nsd)
+    """Flops k_assemble executes per 3D elasticity element, padding included: per
+    quadrature point the Jacobian (nen*nsd^2 multiply-adds) and its inverse (~60), and
+    per 8x8-node tile on or above the diagonal and 4 points nsd^2 m8n8k4 matrix
+    instructions (512 flops each) and, in each of 32 lanes, the physical gradients of
+    two nodes (nsd^2 multiply-adds each) and their weight (nsd)."""
+    geometry = nq * (2 * nen * nsd * nsd + 60)
+    nt = (nen + 7) // 8
+    steps = nt * (nt + 1) // 2 * ((nq + 3) // 4)
+    return geometry + steps * (512 * nsd * nsd + 32 * (4 * nsd * nsd + nsd))
 
 
 def assembly_scatter_bytes_per_element(nen, dpn):
-    """Bytes the element scatter moves per element: every one of its nen^2 node
-    blocks (dpn^2 FP64 values) read and written once."""
-    return nen * nen * dpn * dpn * 8 * 2
+    """Bytes the element scatter sends per element: every one of its nen^2 node blocks
+    (dpn^2 FP64 values) once, stored by the first cell that touches it, added by a
+    reduction in L2 by the others."""
+    return nen * nen * dpn * dpn * 8
 
 
 def fp64_peak_tflops():
@@ -527,9 +529,9 @@ def run_assembly(ctx, dm, phys, nx, reps=5):
             "scatter_bytes": scatter, "scatter_GBs": scatter / t / 1e9,
             "fp64_dgemm_TFLOPs_measured": peak, "frac_of_dgemm": (achieved / peak) if peak else None,
             "executed_frac_of_dgemm": (executed / t / 1e12 / peak) if peak else None,
-            "note": "algorithmic = the B^T D B count; executed = what k_assemble does (node pairs of the upper "
-                    "triangle, 79 flops per pair and point, plus geometry); scatter = read-modify-write of every "
-                    "element block into the value array"}
+            "note": "algorithmic = the B^T D B count; executed = what k_assemble does (8x8-node tiles of the upper "
+                    "triangle by FP64 matrix instructions, padding included, plus geometry); scatter = every "
+                    "element block once into the value array (stores and reductions)"}
 
 
 def run_ilu(ctx, nx=30):

@@ -411,7 +411,9 @@ constexpr int kAsmWarps = 10;  // warps per CTA at most
 // TFLOP/s the matrix instructions reach; 26.2M block updates of 72 bytes, 18.6M of
 // them first touches, 0.37 ms.  What bounds it now is the shared-memory pipe (65 %
 // busy: fragments, and the tiles on their way out) at the 20 warps per SM that the
-// 36 accumulator registers leave.
+// 36 accumulator registers leave; within the 96 registers of that bound 3D elasticity
+// spills a little (144 bytes of stores and 52 of loads in block rows, 252 and 188 in scalar
+// rows).
 template <int NSD, int DPN, int PHYS, bool BCSR>
 __global__ void __launch_bounds__(32 * kAsmWarps, PHYS == YG_ELASTICITY ? 2 : 3)
 k_assemble(const int32_t *__restrict__ order, int ncell, const uint16_t *__restrict__ map,
@@ -847,12 +849,12 @@ static yg_status launch_assemble(yg_context ctx, const ElementGroup &g, yg_dofma
 template <int NSD>
 static yg_status dispatch_physics(yg_context ctx, const ElementGroup &g, yg_dofmap d, int kind, int dpn,
                                   const PhysParams &prm, double *val, int format, double *residual, int wK, int wR) {
-    if (kind == YG_POISSON && dpn == 1) 
+    if (kind == YG_POISSON && dpn == 1)
         return launch_assemble<NSD, 1, YG_POISSON, true>(ctx, g, d, prm, val, residual, wK, wR);
-    if (kind == YG_SUPG && dpn == 1) 
+    if (kind == YG_SUPG && dpn == 1)
         return launch_assemble<NSD, 1, YG_SUPG, true>(ctx, g, d, prm, val, residual, wK, wR);
-    if (kind == YG_ELASTICITY && dpn == NSD) 
-        return format == YG_FORMAT_BCSR || NSD == 1
+    if (kind == YG_ELASTICITY && dpn == NSD)  // (blocks of one entry: the formats are the same)
+        return format == YG_FORMAT_BCSR
                    ? launch_assemble<NSD, NSD, YG_ELASTICITY, true>(ctx, g, d, prm, val, residual, wK, wR)
                    : launch_assemble<NSD, NSD, YG_ELASTICITY, NSD == 1>(ctx, g, d, prm, val, residual, wK, wR);
     return fail(YG_BAD_ARG, "physics %d needs dof_per_node %d (got %d)", kind, kind == YG_ELASTICITY ? NSD : 1, dpn);
