@@ -54,3 +54,38 @@ def test_maps_go_when_they_make_room_and_come_back(mixed):
     for _ in range(20):
         again()
     assert c.memory()[0] == held
+
+
+@pytest.mark.parametrize("phys,fmt", [("poisson", yb.CSR), ("elasticity", yb.BCSR)])
+def test_no_maps_for_cells_that_repeat_a_node(phys, fmt):
+    """Cells that repeat a node have entries that one cell adds to twice, so they never get a
+    map: not even where the pattern was built without room for one and there is room later.
+    Tolerance: four contributions of a cell to an entry, summed in any order (1e-13)."""
+    mesh = meshgen.structured_quad(40, 40, order=meshgen.corner_order(1))
+    mesh["cell_nodes"].reshape(-1, 4)[::7, 2] = mesh["cell_nodes"].reshape(-1, 4)[::7, 3]
+    dpn = 2 if phys == "elasticity" else 1
+    physics = yb.LinearElasticity(2) if dpn == 2 else yb.PoissonEquation(2)
+
+    def system(c):
+        return yb.FESystem(yb.DoFManager(mesh, 1, dpn, ctx=c), 2, format=fmt)
+
+    def values(fe):
+        yb.CGAssembly(physics, fe)
+        return fe.getGlobalTangent().arrays()[2].copy()
+
+    want = values(system(yb.Context(0)))
+    assert np.all(np.isfinite(want))
+    refused = 0
+    for spare in range(8 << 10, 600 << 10, 16 << 10):  # room for less and more than pattern and maps
+        c = yb.Context(0, hbm_budget=64 << 20)
+        fe = system(c)
+        v = yb.DeviceVector(((64 << 20) - c.memory()[0] - spare) // 8, c)
+        try:
+            values(fe)
+        except yb.YafelError as e:
+            assert e.status == _lib.YG_OVER_BUDGET
+            refused += 1
+        del v
+        for _ in range(7):
+            assert np.abs(values(fe) - want).max() <= 1e-13 * np.abs(want).max()
+    assert refused

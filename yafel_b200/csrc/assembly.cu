@@ -873,6 +873,19 @@ static void free_groups(yg_dofmap d) {
     d->groups.clear();
 }
 
+// *odd is set when a cell of `order` does not list exactly nen nodes, each once: no scatter
+// map may be laid out (what k_row_fill finds out on its way when it lays one out).
+__global__ void k_odd_cells(const int32_t *__restrict__ order, int ncell, int nen, const int32_t *__restrict__ off,
+                            const int32_t *__restrict__ el, int32_t *__restrict__ odd) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ncell; t += gridDim.x * blockDim.x) {
+        const int b = off[order[t]];
+        bool bad = off[order[t] + 1] - b != nen;
+        for (int i = 1; i < nen && !bad; ++i)
+            for (int k = 0; k < i && !bad; ++k) bad = el[b + i] == el[b + k];
+        if (bad) *odd = 1;
+    }
+}
+
 // Node graph + element groups for simulation dimension nsd.
 static yg_status build_pattern(yg_dofmap d, int nsd) {
     if (d->pattern_nsd == nsd) return YG_OK;
@@ -979,6 +992,14 @@ static yg_status build_pattern(yg_dofmap d, int nsd) {
         }
         maps.slot = d_slot;
         maps.rank = d_rank;
+    } else {  // (a later assembly may find room for the maps: restore_maps)
+        for (const ElementGroup &gr : d->groups) {
+            const int cells = gr.color_ptr.empty() ? 0 : gr.color_ptr.back();
+            if (cells == 0) continue;
+            k_odd_cells<<<stream_grid(ctx, cells), kThreads, 0, st>>>(gr.d_order, cells, gr.tab.nen, d->d_offsets, d->d_elements,
+                                                                      d_flag);
+            YG_LAUNCHED(ctx);
+        }
     }
     int32_t odd = 0;
     k_row_fill<<<rgrid, kRowWarps * 32, 0, st>>>(nn, d_aptr, d_adj, d->d_offsets, d->d_elements, d_rp64, d->d_nrowptr,
