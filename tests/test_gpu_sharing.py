@@ -1,0 +1,57 @@
+"""A solve that streams its matrix beside a batch of resident systems that another context
+runs over and over: it gets its share of the GPU, and both give the bits they give alone."""
+import threading
+import time
+
+import numpy as np
+import pytest
+
+import yafel_b200 as yb
+from yafel_b200 import workloads
+
+pytestmark = pytest.mark.gpu
+
+
+def test_streaming_solve_beside_resident_batches(ctx):
+    c = yb.Context(0)
+    B, xs = yb.Batch(12, c), []
+    for i in range(12):
+        _, K, b, _ = workloads.assemble(workloads.problem_spec(i, lo=5e3, hi=2e4), c)
+        xs.append(yb.DeviceVector(K.rows(), c))
+        B.add(K, b, xs[-1])
+
+    def batch():
+        for x in xs:
+            x.fill(0.0)
+        B.reset()
+        assert B.run() == 0
+        return [x.numpy() for x in xs]
+
+    _, K, b, _ = workloads.assemble(workloads.problem_spec(3, lo=4e5, hi=4.1e5), ctx)
+    M = yb.JacobiPreconditioner(K)
+
+    def solve():
+        t0 = time.perf_counter()
+        x = yb.solve(K, b, M=M, tol=1e-10)[0]
+        return time.perf_counter() - t0, x.numpy()
+
+    batch_ref, x_ref = batch(), solve()[1]
+    alone = min(solve()[0] for _ in range(3))
+    stop, wrong, runs = [], [], [0]
+
+    def over_and_over():
+        while not stop:
+            if not all(np.array_equal(a, r) for a, r in zip(batch(), batch_ref)):
+                wrong.append(runs[0])
+            runs[0] += 1
+    t = threading.Thread(target=over_and_over)
+    t.start()
+    try:
+        time.sleep(0.1)
+        beside = [solve() for _ in range(4)]
+    finally:
+        stop.append(1)
+        t.join()
+    assert not wrong and runs[0] > 0
+    assert all(np.array_equal(x, x_ref) for _, x in beside)
+    assert min(s for s, _ in beside) <= 4 * alone

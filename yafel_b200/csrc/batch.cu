@@ -144,6 +144,7 @@ struct yg_batch_t {
     cudaGraphExec_t exec = nullptr;
     cudaEvent_t done = nullptr;         // recorded after each launched block
     bool in_flight = false;
+    std::unique_ptr<yg::Beside> beside;  // while a block of the shared kernels is in flight
     // live systems with their own SpMV launches (slot, matrix), and the list the
     // captured graph holds; partial sums of those launches
     std::vector<std::pair<int, yg_matrix>> solo, graph_solo;
@@ -1252,6 +1253,11 @@ constexpr int kResCheck = 16;     // iterations between looks at a due replaceme
 // limit is 2^22, above 4 s: after 4,096 polls each sleeps a microsecond.
 constexpr int kResQueue = 8;
 constexpr int kResRun = 1 << 12;  // iterations of a system per launch
+// Iterations per launch of a run while other contexts solve: their resident kernels wait for
+// the launch where the two find no room beside one another (as above, 3,969 unknowns beside 24 systems:
+// streaming iterations for both 14 / 101, launches of 4,096 iterations 44 / 44, 512 10.5 / 52, 128 5.6 /
+// 60; 60,025 unknowns 46 / 116, then 58 / 58, 25.6 / 126, 19 / 302).
+constexpr int kResTurn = 1 << 9;
 // Blocks of m iterations that a resident system does in one block of the others when a
 // program steps through a batch.  A launch loads every matrix into shared memory again and
 // waits for its longest queue (ms of stepped solves, no resident kernel / 1 block / 2 / 4 / 8: 3
@@ -1650,8 +1656,12 @@ size_t batch_resident_bytes(yg_context ctx) {
 // Launches up to max_its iterations of every live resident system.
 static yg_status launch_resident(yg_batch bt, int max_its) {
     yg_context ctx = bt->ctx;
-    const int ctas = resident_grid(ctx);
-    const size_t most = (size_t)ctas * kResQueue;
+    const size_t most = (size_t)resident_grid(ctx) * kResQueue;
+    // Half the SMs while another context's solve or batch streams: its kernels find room only
+    // between the launches of this one otherwise (403,225 unknowns solved beside 24 systems run
+    // over and over, ms a solve / a run of the 24: streaming iterations for both 215 / 150, all SMs
+    // 1290 / 41, half of them 266 / 84; each alone 165 / 41).
+    const int ctas = Beside::streaming(ctx) ? std::max(std::min(kResMost, resident_grid(ctx)), resident_grid(ctx) / 2) : resident_grid(ctx);
     auto *d_slots = reinterpret_cast<resident::SumSlot *>(ctx->d_slots);
     auto *d_jobs = reinterpret_cast<BatchResident *>(d_slots + 2 * most);
     auto *d_queue = reinterpret_cast<int2 *>(d_jobs + kResJobs);
@@ -1720,7 +1730,10 @@ static yg_status launch_resident(yg_batch bt, int max_its) {
         const void *kern = reinterpret_cast<const void *>(&k_batch_resident);
         const int room = (int)resident_room(ctx);
         YG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
-        YG_TRY(launch_cooperative(ctx, kern, ctas, kResThreads, (size_t)room, args));
+        // (the first CTAs have the systems: the SMs of the others are left to other contexts' launches)
+        int used = ctas;
+        while (used > 1 && plan.queue[used - 1].empty()) --used;
+        YG_TRY(launch_cooperative(ctx, kern, used, kResThreads, (size_t)room, args));
         std::vector<int> rest;
         for (size_t i = 0; i < todo.size(); ++i)
             if (std::find(plan.placed.begin(), plan.placed.end(), (int)i) == plan.placed.end()) rest.push_back(todo[i]);
@@ -2021,10 +2034,12 @@ extern "C" yg_status yg_batch_reset(yg_batch bt, int32_t slot) {
 // host, without waiting.
 static yg_status batch_launch(yg_batch bt, int max_its) {
     yg_context ctx = bt->ctx;
+    bt->beside.reset();
     YG_TRY(launch_resident(bt, max_its));
     bool others = false;
     for (int s = 0; s < bt->capacity; ++s) others = others || (sys_live(bt, s) && !bt->sys[s].resident);
     if (others) {
+        bt->beside.reset(new Beside(ctx, true));
         if (!bt->exec || bt->graph_groups != bt->groups_present || bt->graph_solo != bt->solo) YG_TRY(capture_graph(bt));
         YG_CUDA(cudaGraphLaunch(bt->exec, ctx->stream));
         ctx->launches += bt->graph_kernels;
@@ -2044,6 +2059,7 @@ static yg_status batch_collect(yg_batch bt, int *active_out) {
     yg_context ctx = bt->ctx;
     YG_CUDA(cudaStreamSynchronize(ctx->stream));
     bt->in_flight = false;
+    bt->beside.reset();
     YG_TRY(check_device_error(ctx));
     int active = 0;
     int32_t live = 0;
@@ -2070,9 +2086,11 @@ static yg_status batch_prepare(yg_batch bt) {
 extern "C" yg_status yg_batch_run(yg_batch bt, int32_t max_blocks, int32_t *n_active) {
     if (!bt) return fail(YG_BAD_ARG, "yg_batch_run: NULL batch");
     YG_TRY(batch_prepare(bt));
+    yg_context ctx = bt->ctx;
     int active = 0;
+    // (0: nobody looks at the systems in between; other contexts' solves may wait for the launch)
     for (int blk = 0; max_blocks <= 0 || blk < max_blocks; ++blk) {
-        YG_TRY(batch_launch(bt, max_blocks <= 0 ? kResRun : kResBlocks * bt->m));  // (0: nobody looks at the systems in between)
+        YG_TRY(batch_launch(bt, max_blocks > 0 ? kResBlocks * bt->m : Beside::solving(ctx) ? kResTurn : kResRun));
         YG_TRY(batch_collect(bt, &active));
         if (active == 0) break;
     }

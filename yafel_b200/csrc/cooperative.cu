@@ -30,12 +30,14 @@ struct Device {
     std::mutex m;
     std::vector<cudaEvent_t> spare;  // events of launches that no place holds any more
     std::unique_ptr<SmTurns<Event>> turns;
+    std::atomic<int> solving{0}, streaming{0};
 };
 
-Device &device_of(yg_context ctx) {
+Device &device_at(int device) {
     static auto *all = new Device[64];  // (never destroyed: contexts may outlive static objects)
-    return all[ctx->device & 63];
+    return all[device & 63];
 }
+Device &device_of(yg_context ctx) { return device_at(ctx->device); }
 
 // Runs `launch`, of kernels of up to `blocks` blocks, in its turn.
 template <typename Launch>
@@ -63,6 +65,17 @@ yg_status in_turn(yg_context ctx, int blocks, Launch launch) {
 }
 
 }  // namespace
+
+Beside::Beside(yg_context ctx, bool streams) : device_(ctx->device), streams_(streams) {
+    ++device_at(device_).solving;
+    if (streams_) ++device_at(device_).streaming;
+}
+Beside::~Beside() {
+    --device_at(device_).solving;
+    if (streams_) --device_at(device_).streaming;
+}
+int Beside::solving(yg_context ctx) { return device_of(ctx).solving; }
+int Beside::streaming(yg_context ctx) { return device_of(ctx).streaming; }
 
 yg_status launch_cooperative(yg_context ctx, const void *kern, int grid, int threads, size_t smem, void **args) {
     auto launch = [&]() -> yg_status {

@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <cstdio>
+#include <memory>
 #include <string>
 #include <vector>
 #include <unordered_map>
@@ -209,6 +210,21 @@ yg_status matrix_row_extent(yg_matrix A);
 yg_status launch_cooperative(yg_context ctx, const void *kern, int grid, int threads, size_t smem, void **args);
 yg_status launch_graph(yg_context ctx, cudaGraphExec_t exec, int blocks);
 uint64_t new_stream_number();
+// A solve in progress, or a block of iterations of a batch's shared kernels: what a batch's
+// resident systems look at before they take their SMs for milliseconds.  `streams`: it is
+// one kernel after another, each of which needs room on some SMs.
+class Beside {
+  public:
+    Beside(yg_context ctx, bool streams);
+    ~Beside();
+    Beside(const Beside &) = delete;
+    static int solving(yg_context ctx);    // how many on the context's device
+    static int streaming(yg_context ctx);  // and that stream
+
+  private:
+    int device_;
+    bool streams_;
+};
 // PCG iterations in one cooperative kernel (pcg_resident.cu)
 yg_status pcg_resident_fits(yg_matrix A, bool f32, bool jacobi, bool *fits);
 yg_status pcg_resident_launch(yg_matrix A, bool f32, const double *dinv, const double *b, double *x, double *r,

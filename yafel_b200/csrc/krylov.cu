@@ -436,6 +436,7 @@ static yg_status pcg_core(yg_matrix A, yg_precond M, const double *b, double *x,
     double *P = ctx->d_partials;  // [0,2G): p.q ; [2G,4G): r.z/r.r pairs ; [4G, 7G): init triples
     KrylovScalars *S = ctx->d_scalars;
     cudaStream_t st = ctx->stream;
+    Beside beside(ctx, !w.zp);
     // the FP32 direction copy serves the FP32-value iteration SpMV only; so does
     // the row-sum correction of the FP32 values (the operator A32 x + C x_own)
     const bool f32 = precision == YG_PREC_MIXED || precision == YG_PREC_MIXED_IR;
