@@ -153,7 +153,9 @@ struct yg_batch_t {
     int64_t solo_bytes = kSoloSpmvBytes;  // threshold for systems added from now on (0: none)
     cudaGraph_t graph = nullptr;
     int64_t graph_kernels = 0;
-    std::vector<BatchScal> h_scal;
+    // (pinned: a copy to other memory keeps the host here until the block is done, and with it a
+    // lock of the driver that other contexts' solves need)
+    BatchScal *h_scal = nullptr;
 };
 
 namespace yg {
@@ -1848,10 +1850,17 @@ extern "C" yg_status yg_batch_create(yg_context ctx, int32_t capacity, yg_batch 
         yg_batch_destroy(bt);
         return fail(YG_CUDA_ERROR, "yg_batch_create: event creation failed");
     }
-    std::vector<BatchScal> init(capacity);
-    for (auto &c : init) c.flag = BF_EMPTY;
-    bt->h_scal = init;
-    cudaMemcpy(bt->d_scal, init.data(), sizeof(BatchScal) * capacity, cudaMemcpyHostToDevice);
+    if (cudaMallocHost(&bt->h_scal, sizeof(BatchScal) * capacity) != cudaSuccess) {
+        cudaGetLastError();
+        bt->h_scal = nullptr;
+        yg_batch_destroy(bt);
+        return fail(YG_OUT_OF_MEMORY, "yg_batch_create: no pinned memory for the systems' states");
+    }
+    for (int32_t s = 0; s < capacity; ++s) {
+        bt->h_scal[s] = BatchScal{};
+        bt->h_scal[s].flag = BF_EMPTY;
+    }
+    cudaMemcpy(bt->d_scal, bt->h_scal, sizeof(BatchScal) * capacity, cudaMemcpyHostToDevice);
     cudaMemset(bt->d_ranges, 0, sizeof(int32_t) * kRanges);
     YG_CUDA(cudaGetLastError());
     *out = bt;
@@ -1869,6 +1878,7 @@ extern "C" yg_status yg_batch_destroy(yg_batch bt) {
                     (void *)bt->d_solo_part})
         dev_free(bt->ctx, p);
     if (bt->done) cudaEventDestroy(bt->done);
+    if (bt->h_scal) cudaFreeHost(bt->h_scal);
     delete bt;
     return YG_OK;
 }
@@ -2024,7 +2034,7 @@ extern "C" yg_status yg_batch_reset(yg_batch bt, int32_t slot) {
         sc.resident = bt->sys[s].resident > 0;
         bt->h_scal[s] = sc;
     }
-    YG_CUDA(cudaMemcpy(bt->d_scal + s0, bt->h_scal.data() + s0, sizeof(BatchScal) * (s1 - s0), cudaMemcpyHostToDevice));
+    YG_CUDA(cudaMemcpy(bt->d_scal + s0, bt->h_scal + s0, sizeof(BatchScal) * (s1 - s0), cudaMemcpyHostToDevice));
     bt->dirty = true;
     return YG_OK;
 }
@@ -2046,7 +2056,7 @@ static yg_status batch_launch(yg_batch bt, int max_its) {
     } else {
         launch_verify(bt);
     }
-    YG_CUDA(cudaMemcpyAsync(bt->h_scal.data(), bt->d_scal, sizeof(BatchScal) * bt->capacity, cudaMemcpyDeviceToHost,
+    YG_CUDA(cudaMemcpyAsync(bt->h_scal, bt->d_scal, sizeof(BatchScal) * bt->capacity, cudaMemcpyDeviceToHost,
                             ctx->stream));
     YG_CUDA(cudaEventRecord(bt->done, ctx->stream));
     bt->in_flight = true;
@@ -2075,6 +2085,7 @@ static yg_status batch_collect(yg_batch bt, int *active_out) {
 }
 
 static yg_status batch_prepare(yg_batch bt) {
+    if (bt->in_flight) YG_CUDA(cudaStreamSynchronize(bt->ctx->stream));  // (a block that was not waited for: its states count)
     if (bt->dirty) YG_TRY(rebuild_items(bt));
     launch_verify(bt);  // initialise systems added since the last run
     return YG_OK;
@@ -2128,6 +2139,7 @@ extern "C" yg_status yg_batch_stats(yg_batch bt, int32_t slot, yg_solve_stats *o
 extern "C" yg_status yg_batch_tune(yg_batch bt) {
     if (!bt) return fail(YG_BAD_ARG, "yg_batch_tune: NULL batch");
     yg_context ctx = bt->ctx;
+    YG_CUDA(cudaStreamSynchronize(ctx->stream));
     // initialise p / ph from a verification pass so the SpMV reads defined data
     YG_TRY(rebuild_items(bt));
     launch_verify(bt);
