@@ -95,3 +95,40 @@ def test_small_solves_beside_small_batches(ctx):
     assert all(np.array_equal(x, x_ref) for _, x in beside)
     # (1.7 with streaming iterations for both, 5.3 with a batch that keeps the driver waiting)
     assert np.median([s for s, _ in beside]) <= 2.5 * alone
+
+
+@pytest.mark.parametrize("rows,limit", [(4e5, 6.0), (4e3, 8.0)])
+def test_solves_beside_resident_solves_on_all_sms(ctx, rows, limit):
+    """A program that solves a system in the shared memory of all SMs over and over takes turns
+    with another's solves, streaming ones and small ones."""
+    c = yb.Context(0)
+    _, Kw, bw, _ = workloads.assemble(workloads.problem_spec(3, lo=1.2e5, hi=1.21e5), c)
+    Mw = yb.JacobiPreconditioner(Kw)
+    _, K, b, _ = workloads.assemble(workloads.problem_spec(3, lo=rows, hi=1.01 * rows), ctx)
+    M = yb.JacobiPreconditioner(K)
+
+    def solve():
+        t0 = time.perf_counter()
+        x = yb.solve(K, b, M=M, tol=1e-10)[0]
+        return time.perf_counter() - t0, x.numpy()
+
+    x_ref, wide_ref = solve()[1], yb.solve(Kw, bw, M=Mw, tol=1e-10)[0].numpy()
+    alone = np.median([solve()[0] for _ in range(5)])
+    stop, wrong = [], []
+
+    def over_and_over():
+        while not stop:
+            if not np.array_equal(yb.solve(Kw, bw, M=Mw, tol=1e-10)[0].numpy(), wide_ref):
+                wrong.append(1)
+    t = threading.Thread(target=over_and_over)
+    t.start()
+    try:
+        time.sleep(0.1)
+        beside = [solve() for _ in range(3 if rows > 1e5 else 40)]
+    finally:
+        stop.append(1)
+        t.join()
+    assert not wrong
+    assert all(np.array_equal(x, x_ref) for _, x in beside)
+    # (2.2 and about 3; 117 and 15 without turns)
+    assert np.mean([s for s, _ in beside]) <= limit * alone

@@ -1482,6 +1482,7 @@ extern "C" yg_status yg_dofmap_get(yg_dofmap d, double *dof_nodes_xyz, int32_t *
 extern "C" yg_status yg_assemble(yg_dofmap d, const yg_physics *physics, uint32_t requirements, int32_t format,
                                  yg_matrix *K, yg_vector residual) {
     if (!d || !physics) return fail(YG_BAD_ARG, "yg_assemble: NULL argument");
+    Beside beside(d->ctx, Beside::kStreams);
     const int nsd = physics->nsd;
     if (nsd < 1 || nsd > 3) return fail(YG_BAD_ARG, "physics nsd must be 1..3");
     if (format != YG_FORMAT_CSR && format != YG_FORMAT_BCSR) return fail(YG_BAD_ARG, "unknown format %d", format);

@@ -144,7 +144,7 @@ struct yg_batch_t {
     cudaGraphExec_t exec = nullptr;
     cudaEvent_t done = nullptr;         // recorded after each launched block
     bool in_flight = false;
-    std::unique_ptr<yg::Beside> beside;  // while a block of the shared kernels is in flight
+    bool shared_in_flight = false;       // the block has systems of the shared kernels
     // live systems with their own SpMV launches (slot, matrix), and the list the
     // captured graph holds; partial sums of those launches
     std::vector<std::pair<int, yg_matrix>> solo, graph_solo;
@@ -2044,12 +2044,10 @@ extern "C" yg_status yg_batch_reset(yg_batch bt, int32_t slot) {
 // host, without waiting.
 static yg_status batch_launch(yg_batch bt, int max_its) {
     yg_context ctx = bt->ctx;
-    bt->beside.reset();
     YG_TRY(launch_resident(bt, max_its));
     bool others = false;
     for (int s = 0; s < bt->capacity; ++s) others = others || (sys_live(bt, s) && !bt->sys[s].resident);
     if (others) {
-        bt->beside.reset(new Beside(ctx, true));
         if (!bt->exec || bt->graph_groups != bt->groups_present || bt->graph_solo != bt->solo) YG_TRY(capture_graph(bt));
         YG_CUDA(cudaGraphLaunch(bt->exec, ctx->stream));
         ctx->launches += bt->graph_kernels;
@@ -2060,6 +2058,7 @@ static yg_status batch_launch(yg_batch bt, int max_its) {
                             ctx->stream));
     YG_CUDA(cudaEventRecord(bt->done, ctx->stream));
     bt->in_flight = true;
+    bt->shared_in_flight = others;
     return YG_OK;
 }
 
@@ -2067,9 +2066,11 @@ static yg_status batch_launch(yg_batch bt, int max_its) {
 // work tables once a quarter of the vector items is idle.
 static yg_status batch_collect(yg_batch bt, int *active_out) {
     yg_context ctx = bt->ctx;
-    YG_CUDA(cudaStreamSynchronize(ctx->stream));
-    bt->in_flight = false;
-    bt->beside.reset();
+    {
+        std::unique_ptr<Beside> beside(bt->shared_in_flight ? new Beside(ctx, Beside::kStreams) : nullptr);
+        YG_CUDA(cudaStreamSynchronize(ctx->stream));
+    }
+    bt->in_flight = bt->shared_in_flight = false;
     YG_TRY(check_device_error(ctx));
     int active = 0;
     int32_t live = 0;
@@ -2101,7 +2102,7 @@ extern "C" yg_status yg_batch_run(yg_batch bt, int32_t max_blocks, int32_t *n_ac
     int active = 0;
     // (0: nobody looks at the systems in between; other contexts' solves may wait for the launch)
     for (int blk = 0; max_blocks <= 0 || blk < max_blocks; ++blk) {
-        YG_TRY(batch_launch(bt, max_blocks > 0 ? kResBlocks * bt->m : Beside::solving(ctx) ? kResTurn : kResRun));
+        YG_TRY(batch_launch(bt, max_blocks > 0 ? kResBlocks * bt->m : Beside::others(ctx, 0) ? kResTurn : kResRun));
         YG_TRY(batch_collect(bt, &active));
         if (active == 0) break;
     }

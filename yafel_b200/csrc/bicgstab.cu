@@ -271,7 +271,7 @@ yg_status solve_bicgstab(yg_matrix A, yg_precond M, yg_vector bv, yg_vector xv, 
     yg_solve_opts o = opts ? *opts : yg_solve_opts{YG_CRIT_REFERENCE, YG_PREC_FP64, 1e-14, 0, 0, 0};
     if (o.precision != YG_PREC_FP64) return fail(YG_UNSUPPORTED, "BiCGSTAB supports FP64 only");
     if (M && !precond_fusable(M)) return fail(YG_UNSUPPORTED, "BiCGSTAB takes Jacobi or identity preconditioning");
-    Beside beside(ctx, true);
+    Beside beside(ctx, Beside::kStreams);
     const double *dinv = precond_dinv(M);
     const int64_t maxiter = o.maxiter > 0 ? o.maxiter : 100 * n + 1000;
     const int G = ctx->reduce_blocks;

@@ -251,6 +251,7 @@ int stream_grid(yg_context ctx, int64_t n) {
 }
 
 yg_status vector_dot(yg_context ctx, const double *a, const double *b, int64_t n, double *out) {
+    Beside beside(ctx, Beside::kStreams);
     int g = stream_grid(ctx, n);
     if (g > kMaxReduceBlocks) g = kMaxReduceBlocks;
     k_dot_partials<<<g, kThreads, 0, ctx->stream>>>(a, b, n, ctx->d_partials);
@@ -377,6 +378,7 @@ extern "C" yg_status yg_context_destroy(yg_context ctx) {
 
 extern "C" yg_status yg_context_synchronize(yg_context ctx) {
     if (!ctx) return fail(YG_BAD_ARG, "NULL context");
+    Beside beside(ctx, Beside::kStreams);
     YG_CUDA(cudaStreamSynchronize(ctx->stream));
     return check_device_error(ctx);
 }
@@ -435,6 +437,7 @@ extern "C" int64_t yg_vector_size(yg_vector v) { return v ? v->n : -1; }
 
 extern "C" yg_status yg_vector_upload(yg_vector v, const double *host, int64_t n) {
     if (!v || (!host && n) || n != v->n) return fail(YG_BAD_ARG, "yg_vector_upload: size %lld != %lld", (long long)n, v ? (long long)v->n : -1LL);
+    Beside beside(v->ctx, Beside::kStreams);
     YG_CUDA(cudaMemcpyAsync(v->d, host, sizeof(double) * n, cudaMemcpyHostToDevice, v->ctx->stream));
     YG_CUDA(cudaStreamSynchronize(v->ctx->stream));
     return YG_OK;
@@ -442,6 +445,7 @@ extern "C" yg_status yg_vector_upload(yg_vector v, const double *host, int64_t n
 
 extern "C" yg_status yg_vector_download(yg_vector v, double *host, int64_t n) {
     if (!v || (!host && n) || n != v->n) return fail(YG_BAD_ARG, "yg_vector_download: size mismatch");
+    Beside beside(v->ctx, Beside::kStreams);
     YG_CUDA(cudaMemcpyAsync(host, v->d, sizeof(double) * n, cudaMemcpyDeviceToHost, v->ctx->stream));
     YG_CUDA(cudaStreamSynchronize(v->ctx->stream));
     return check_device_error(v->ctx);
@@ -617,6 +621,7 @@ extern "C" yg_status yg_spmv_ex(yg_matrix A, yg_vector x, yg_vector y, int32_t p
                     (long long)A->cols(), (long long)x->n, (long long)y->n);
     if (precision != YG_PREC_FP64 && precision != YG_PREC_MIXED && precision != YG_SPMV_MIXED_CORRECTED)
         return fail(YG_BAD_ARG, "yg_spmv: precision %d is not an SpMV precision", (int)precision);
+    Beside beside(A->ctx, Beside::kStreams);
     const bool corrected = precision == YG_SPMV_MIXED_CORRECTED;
     if (corrected) precision = YG_PREC_MIXED;
     if (precision == YG_PREC_MIXED && !A->d_val32) YG_TRY(yg_matrix_make_fp32(A));

@@ -4,7 +4,9 @@
 #include "sm_turns.h"
 
 #include <atomic>
+#include <chrono>
 #include <mutex>
+#include <thread>
 
 namespace yg {
 
@@ -14,6 +16,8 @@ uint64_t new_stream_number() {
 }
 
 namespace {
+
+using Clock = std::chrono::steady_clock;
 
 struct Event {
     cudaEvent_t e = nullptr;
@@ -30,14 +34,19 @@ struct Device {
     std::mutex m;
     std::vector<cudaEvent_t> spare;  // events of launches that no place holds any more
     std::unique_ptr<SmTurns<Event>> turns;
-    std::atomic<int> solving{0}, streaming{0};
+    std::atomic<int> calls[3]{};  // in progress, by Beside::Kind
+    // the two contexts whose calls ended last, the later one first
+    std::mutex ended_m;
+    struct {
+        uint64_t stream = 0;
+        Clock::time_point at{};
+    } ended[2];
 };
 
-Device &device_at(int device) {
+Device &device_of(yg_context ctx) {
     static auto *all = new Device[64];  // (never destroyed: contexts may outlive static objects)
-    return all[device & 63];
+    return all[ctx->device & 63];
 }
-Device &device_of(yg_context ctx) { return device_at(ctx->device); }
 
 // Runs `launch`, of kernels of up to `blocks` blocks, in its turn.
 template <typename Launch>
@@ -66,16 +75,31 @@ yg_status in_turn(yg_context ctx, int blocks, Launch launch) {
 
 }  // namespace
 
-Beside::Beside(yg_context ctx, bool streams) : device_(ctx->device), streams_(streams) {
-    ++device_at(device_).solving;
-    if (streams_) ++device_at(device_).streaming;
-}
+Beside::Beside(yg_context ctx, Kind kind) : ctx_(ctx), kind_(kind) { ++device_of(ctx).calls[kind]; }
 Beside::~Beside() {
-    --device_at(device_).solving;
-    if (streams_) --device_at(device_).streaming;
+    Device &d = device_of(ctx_);
+    std::lock_guard<std::mutex> hold(d.ended_m);
+    if (d.ended[0].stream != ctx_->stream_number) d.ended[1] = d.ended[0];
+    d.ended[0] = {ctx_->stream_number, Clock::now()};
+    --d.calls[kind_];
 }
-int Beside::solving(yg_context ctx) { return device_of(ctx).solving; }
-int Beside::streaming(yg_context ctx) { return device_of(ctx).streaming; }
+int Beside::streaming(yg_context ctx) { return device_of(ctx).calls[kStreams]; }
+int Beside::not_wide(yg_context ctx) { return streaming(ctx) + device_of(ctx).calls[kNarrow]; }
+bool Beside::others(yg_context ctx, int own) {
+    Device &d = device_of(ctx);
+    if (not_wide(ctx) + d.calls[kWide] > own) return true;
+    std::lock_guard<std::mutex> hold(d.ended_m);
+    const auto &last = d.ended[d.ended[0].stream == ctx->stream_number];
+    return last.stream && Clock::now() - last.at < std::chrono::milliseconds(10);
+}
+void Beside::yield(yg_context ctx, double ms) {
+    const auto end = Clock::now() + std::chrono::duration<double, std::milli>(ms);
+    auto seen = Clock::now();
+    for (auto now = seen; now < end && now - seen < std::chrono::microseconds(100); now = Clock::now()) {
+        if (not_wide(ctx)) seen = now;  // (a program's next call follows the last one within microseconds)
+        std::this_thread::sleep_for(std::chrono::microseconds(20));
+    }
+}
 
 yg_status launch_cooperative(yg_context ctx, const void *kern, int grid, int threads, size_t smem, void **args) {
     auto launch = [&]() -> yg_status {

@@ -210,23 +210,30 @@ yg_status matrix_row_extent(yg_matrix A);
 yg_status launch_cooperative(yg_context ctx, const void *kern, int grid, int threads, size_t smem, void **args);
 yg_status launch_graph(yg_context ctx, cudaGraphExec_t exec, int blocks);
 uint64_t new_stream_number();
-// A solve in progress, or a block of iterations of a batch's shared kernels: what a batch's
-// resident systems look at before they take their SMs for milliseconds.  `streams`: it is
-// one kernel after another, each of which needs room on some SMs.
+// A call in progress that another context's kernels must not hold up for long: resident
+// solves and batches look at it before they take their SMs for milliseconds.  It waits for
+// one kernel after another, each of which needs room on some SMs (kStreams), or is a resident
+// solve that leaves at least half of the SMs free (kNarrow) or does not (kWide).
 class Beside {
   public:
-    Beside(yg_context ctx, bool streams);
+    enum Kind { kStreams, kNarrow, kWide };
+    Beside(yg_context ctx, Kind kind);
     ~Beside();
     Beside(const Beside &) = delete;
-    static int solving(yg_context ctx);    // how many on the context's device
-    static int streaming(yg_context ctx);  // and that stream
+    static int streaming(yg_context ctx);  // how many of the first kind on the context's device
+    static int not_wide(yg_context ctx);   // and of the first two
+    // whether another context has a call in progress, beside `own` of this one, or had one
+    // within 10 ms (a program that has just returned from one is about to make the next)
+    static bool others(yg_context ctx, int own);
+    static void yield(yg_context ctx, double ms);  // waits as long at most, while there are any not wide
 
   private:
-    int device_;
-    bool streams_;
+    yg_context ctx_;
+    Kind kind_;
 };
 // PCG iterations in one cooperative kernel (pcg_resident.cu)
 yg_status pcg_resident_fits(yg_matrix A, bool f32, bool jacobi, bool *fits);
+int pcg_resident_blocks(yg_matrix A, bool f32, bool jacobi);
 yg_status pcg_resident_launch(yg_matrix A, bool f32, const double *dinv, const double *b, double *x, double *r,
                               double *p, double *zp, int max_its, int check, double rr_replace);
 // batch engine, host side (batch.cu)

@@ -418,6 +418,15 @@ struct SpmvProfile {
     }
 };
 
+// Iterations per launch of a resident solve on more than half of the SMs while other
+// contexts' calls are in progress, and the longest it then waits between two launches (it
+// waits as long as the launch took, while one of those calls is not a solve of its kind).  A
+// program that solves over and over beside one that solves 120,409 unknowns over and over, ms
+// a solve of each, streaming iterations for both / no turns / turns: 403,225 unknowns (165 alone)
+// 191, 95 / 19,000, 33 / 354, 63; 3,969 (2.4 alone) 10.2, 56 / 36, 35 / 7.7, 48.
+constexpr int kTurn = 1 << 9;
+constexpr double kTurnMost = 10;  // ms
+
 static yg_status pcg_core(yg_matrix A, yg_precond M, const double *b, double *x, int precision, int criterion,
                           double tol, int64_t maxiter, int check_every, Work &w, int64_t *iters, int *flag_out,
                           SpmvProfile *prof = nullptr, int64_t *replacements = nullptr) {
@@ -436,7 +445,8 @@ static yg_status pcg_core(yg_matrix A, yg_precond M, const double *b, double *x,
     double *P = ctx->d_partials;  // [0,2G): p.q ; [2G,4G): r.z/r.r pairs ; [4G, 7G): init triples
     KrylovScalars *S = ctx->d_scalars;
     cudaStream_t st = ctx->stream;
-    Beside beside(ctx, !w.zp);
+    const bool wide = w.zp && 2 * pcg_resident_blocks(A, precision != YG_PREC_FP64, dinv != nullptr) > ctx->num_sms;
+    Beside beside(ctx, wide ? Beside::kWide : w.zp ? Beside::kNarrow : Beside::kStreams);
     // the FP32 direction copy serves the FP32-value iteration SpMV only; so does
     // the row-sum correction of the FP32 values (the operator A32 x + C x_own)
     const bool f32 = precision == YG_PREC_MIXED || precision == YG_PREC_MIXED_IR;
@@ -518,12 +528,15 @@ static yg_status pcg_core(yg_matrix A, yg_precond M, const double *b, double *x,
         // rows 12.2 and 11.9).  The event pairs of a profile belong to the graph.
         const int64_t direct_its = prof && prof->on ? 0 : 2 * check_every;
         double rr_last = hs.rr;  // r.r at the last replacement
+        double rr_replace = 1e-2 * hs.rr;
         int false_stops = 0;
         for (;;) {
             int64_t before = hs.iter;
+            const bool turn = wide && Beside::others(ctx, 1);
+            const auto t0 = std::chrono::steady_clock::now();
             if (w.zp) {
-                YG_TRY(pcg_resident_launch(A, f32, dinv, b, x, w.r, w.p, w.zp, 1 << 12, check_every,
-                                           reliable ? 1e-2 * rr_last : 0.0));
+                YG_TRY(pcg_resident_launch(A, f32, dinv, b, x, w.r, w.p, w.zp, turn ? kTurn : 1 << 12, check_every,
+                                           reliable ? rr_replace : 0.0));
             } else if (before < direct_its) {
                 for (int it = 0; it < check_every && before + it < maxiter; ++it) YG_TRY(one(it & 1));
                 YG_CUDA(cudaGetLastError());
@@ -534,9 +547,11 @@ static yg_status pcg_core(yg_matrix A, yg_precond M, const double *b, double *x,
             }
             YG_TRY(read_scalars(ctx, &hs));
             if (w.zp && hs.replaced) {
-                rr_last = 1e2 * hs.rr_replace;
+                rr_replace = hs.rr_replace;
                 if (replacements) *replacements += hs.replaced;
             }
+            if (turn && hs.flag == FLAG_RUN)
+                Beside::yield(ctx, std::min(kTurnMost, std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count()));
             if (prof) YG_TRY(prof->collect(hs.iter - before));
             if (hs.flag == FLAG_RUN) {
                 // replace once the recursive residual fell 10x since the last time
@@ -552,6 +567,7 @@ static yg_status pcg_core(yg_matrix A, yg_precond M, const double *b, double *x,
                 YG_TRY(replace(1));
                 YG_TRY(read_scalars(ctx, &hs));
                 rr_last = hs.rr;
+                rr_replace = 1e-2 * hs.rr;
                 if (sqrt(hs.rr) <= tol * sqrt(hs.bb) || hs.iter >= maxiter || ++false_stops > 20) {
                     hs.flag = (sqrt(hs.rr) <= tol * sqrt(hs.bb)) ? FLAG_CONVERGED
                                                                   : (hs.iter >= maxiter ? FLAG_MAXITER : FLAG_CONVERGED);

@@ -101,7 +101,7 @@ static int64_t resident_smem(yg_matrix A, bool f32, bool jacobi, int G) {
 // 527, 1007, 2000, 2359; 30,258 of order-2 plane elasticity 32, 49, 62, 58 -> 53 whatever the
 // threads; 150,000 of order-2 Poisson 15, 22, 27, 26 -> 22).  Half the SMs for the second
 // would let two run at once, 102 a second, but a solve alone takes 1.9 % longer.
-static int resident_blocks(yg_matrix A, bool f32, bool jacobi) {
+int pcg_resident_blocks(yg_matrix A, bool f32, bool jacobi) {
     yg_context ctx = A->ctx;
     const double entries = (double)A->nnzb * A->block * A->block;
     const int most = (int)std::min<int64_t>(ctx->num_sms, A->nbrows);
@@ -121,7 +121,7 @@ yg_status pcg_resident_fits(yg_matrix A, bool f32, bool jacobi, bool *fits) {
     const int64_t total = A->nnzb * bc + A->nbrows * rc, room = (int64_t)ctx->smem_optin - kStaticSmem;
     if (total / ctx->num_sms > room) return YG_OK;
     YG_TRY(matrix_row_extent(A));
-    *fits = resident_smem(A, f32, jacobi, resident_blocks(A, f32, jacobi)) <= room;
+    *fits = resident_smem(A, f32, jacobi, pcg_resident_blocks(A, f32, jacobi)) <= room;
     return YG_OK;
 }
 
@@ -154,7 +154,7 @@ yg_status pcg_resident_launch(yg_matrix A, bool f32, const double *dinv, const d
     a.rr_replace = rr_replace;
     a.val64 = A->d_val;
     a.b = b;
-    const int G = resident_blocks(A, f32, dinv != nullptr);
+    const int G = pcg_resident_blocks(A, f32, dinv != nullptr);
     const double mean = (double)A->nnzb / A->nbrows;
     const int64_t rows = (A->nbrows + G - 1) / G;
     const int threads = rows * (mean > 8 ? 8 : 4) > 512 ? 512 : 256;

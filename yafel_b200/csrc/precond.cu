@@ -525,6 +525,7 @@ using namespace yg;
 
 extern "C" yg_status yg_precond_create(yg_matrix A, int32_t kind, yg_precond *out) {
     if (!A || !out) return fail(YG_BAD_ARG, "yg_precond_create: NULL argument");
+    Beside beside(A->ctx, Beside::kStreams);
     if (A->rows() != A->cols()) return fail(YG_BAD_ARG, "preconditioner needs a square matrix");
     *out = nullptr;
     auto *M = new yg_precond_t();
