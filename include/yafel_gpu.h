@@ -356,7 +356,8 @@ typedef struct yg_solve_opts {
     double tol;         /* see criterion */
     int64_t maxiter;    /* 0 = the reference's default (N for CG) */
     int32_t check_every;/* iterations between host convergence checks (0 = automatic) */
-    int32_t profile;    /* 1: time every SpMV of the iteration with CUDA events (stats.spmv_*) */
+    int32_t profile;    /* 1: time every SpMV of the iteration with CUDA events (stats.spmv_*); such a solve
+                           streams its matrix, also one that would fit the SMs' shared memory */
 } yg_solve_opts;
 typedef struct yg_solve_stats {
     int64_t iterations;       /* Krylov iterations (inner iterations summed for MIXED) */

@@ -743,7 +743,8 @@ class ILUPreconditioner(_Precond):
 def solve(A, b, x0=None, M=None, method="cg", criterion=CRIT_RELRES, tol=1e-10, maxiter=0,
           precision=PREC_FP64, check_every=0, raise_on_failure=False, profile=False):
     """Solve on the GPU and return (x, stats).  b and x0 may be host arrays or
-    DeviceVectors; x is a DeviceVector."""
+    DeviceVectors; x is a DeviceVector.  profile: time the iteration's SpMVs (a
+    profiled solve streams its matrix, also one that would fit the SMs' shared memory)."""
     ctx = A.ctx
     bd, _ = _as_device(b, ctx)
     if x0 is None:

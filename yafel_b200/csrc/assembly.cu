@@ -409,9 +409,9 @@ constexpr int kAsmWarps = 10;  // warps per CTA at most
 // 0.84 ms, scalar 37^3 Q2 2.23 -> 0.71 ms, 60^3 Q1 1.53 -> 0.25 ms, 200^2 Q2 2x2 blocks
 // 0.33 -> 0.13 ms.  Floors of the first: 161k FMA per cell, 0.16 ms at the 37
 // TFLOP/s the matrix instructions reach; 26.2M block updates of 72 bytes, 18.6M of
-// them first touches, 0.37 ms.  What bounds it now is the shared-memory pipe (65 %
-// busy: fragments, and the tiles on their way out) at the 20 warps per SM that the
-// 36 accumulator registers leave; within the 96 registers of that bound 3D elasticity
+// them first touches, 0.37 ms.  What bounds it now is latency at the 20 warps per SM that
+// the 36 accumulator registers leave, with L1/TEX 62 % busy (fragments, and the tiles on
+// their way out; 30^3, one colour); within the 96 registers of that bound 3D elasticity
 // spills a little (144 bytes of stores and 52 of loads in block rows, 252 and 188 in scalar
 // rows).
 template <int NSD, int DPN, int PHYS, bool BCSR>
