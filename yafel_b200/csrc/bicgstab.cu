@@ -15,7 +15,10 @@
 // evaluated between runs of iterations, at exactly those.  A run of 32 even-numbered
 // iterations replays a graph; what is left over, and the first two runs of the
 // relative criterion, are launched kernel by kernel (a solve of 2 iterations took
-// 0.70 ms with its graph and 0.25 without at 27,783 rows).
+// 0.70 ms with its graph and 0.25 without at 27,783 rows; at 80,802 one of 24 1.45 and 1.20, one of
+// 40, which pays for both, 2.06 and 2.17, and from 64 on the two are even).  Graphs of 4
+// iterations instead of 16, cheaper to make, took 0.1 ms off the 40 but added up to 20 % to
+// solves of 2,000 iterations at 10,201 rows (33 -> 40 ms).
 #include "internal.h"
 #include "device_common.cuh"
 
